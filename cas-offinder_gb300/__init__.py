@@ -44,7 +44,7 @@ EXPORTS = [
     "cof_router_open", "cof_router_add_genome", "cof_router_drop_genome", "cof_router_genomes", "cof_router_submit",
     "cof_router_wait", "cof_router_release", "cof_router_last_error", "cof_router_close",
     "cof_gzip_open", "cof_gzip_write", "cof_gzip_write_fn", "cof_gzip_close",
-    "cofx_synth_record", "cofx_mismatch_table", "cofx_bs_programs", "cofx_genome_text",
+    "cofx_synth_record", "cofx_mismatch_table", "cofx_bs_programs", "cofx_screen_plan", "cofx_genome_text",
 ]
 
 # cof_write_fn: int (*)(void* ctx, const char* data, size_t len)
@@ -150,6 +150,7 @@ def lib():
             "cof_timer_stop": (c.c_int, [vp, c.POINTER(c.c_double)]),
             "cofx_mismatch_table": (None, [vp]),
             "cofx_bs_programs": (c.c_int, [c.c_char_p, sz, vp, vp, sz, vp, sz, vp, sz]),
+            "cofx_screen_plan": (c.c_int, [c.c_char_p, sz, c.c_int, vp, vp, sz, vp, sz]),
             "cofx_genome_text": (c.c_int, [c.c_char_p, vp, u64, c.POINTER(u64)]),
             "cofx_synth_record": (u64, [u64, u32, u64, c.c_double, c.c_double, u32, c.c_double, u32, u32, vp]),
         }
@@ -209,6 +210,25 @@ def bs_programs(text):
     variants = [(ln.split("\t")[0], int(ln.split("\t")[1])) for ln in keys.raw[:kb].decode().splitlines()]
     return {"chunks": chunks, "m": m, "slots": slots, "row": row, "prog": prog, "pgid": pgid, "variants": variants,
             "narrow": bool(narrow)}
+
+
+def screen_plan(text, level=-1):
+    """The table screen planned for one input file (test hook), or None where
+    none is: dict with its geometry, the records by class and `first`."""
+    raw = text.encode() if isinstance(text, str) else bytes(text)
+    info = np.zeros(27, dtype=np.uint32)
+    if lib().cofx_screen_plan(raw, len(raw), level, _ptr(info), None, 0, None, 0) != 0:
+        raise CofError(4, "parse error")
+    x = [int(v) for v in info]
+    if not x[0]:
+        return None
+    out = dict(zip(("entries", "bits", "fields", "top", "words", "degenerate", "variants", "record_words"), x[19:]))
+    out.update(L=x[1], K=x[2], a=x[3:7], q=x[7:11], base=x[11:15], cap=x[15:19])
+    rec = np.zeros(out["variants"] * out["record_words"], dtype=np.uint32)
+    first = np.zeros(out["words"] * (out["fields"] + 1), dtype=np.uint32)
+    lib().cofx_screen_plan(raw, len(raw), level, _ptr(info), _ptr(rec), rec.size, _ptr(first), first.size)
+    out.update(records=rec.reshape(-1, out["record_words"]), first=first.reshape(out["words"], -1))
+    return out
 
 
 def plane_words(n):
@@ -418,7 +438,8 @@ class CasOFFinder:
         return mm_loci[:k].copy(), mm_count[:k].copy(), direction[:k].tobytes()
 
     def set_comparer(self, kind):
-        """0 auto (bit-sliced when it fits), 1 popcount, 2 bit-sliced."""
+        """0 auto (table screen where it pays, else bit-sliced when it fits), 1
+        popcount, 2 bit-sliced when it fits."""
         self._check(self._L.cof_set_comparer(self._h, kind))
 
     def set_autotune(self, on=True):
@@ -434,7 +455,7 @@ class CasOFFinder:
     def comparer_info(self):
         k, sl = ctypes.c_int(), ctypes.c_int()
         self._check(self._L.cof_comparer_info(self._h, ctypes.byref(k), ctypes.byref(sl)))
-        return {"kind": {1: "popcount", 2: "bit-sliced"}[k.value], "slots": sl.value}
+        return {"kind": {1: "popcount", 2: "bit-sliced", 3: "screen"}[k.value], "slots": sl.value}
 
     # instrumentation
     def set_profiling(self, on=True):

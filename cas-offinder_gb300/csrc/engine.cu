@@ -416,8 +416,25 @@ void pinned_release(cof_handle* h, void* p, size_t cap) {
   }
 }
 
-void build_group_host(bool force_popc, PatternGroup& g, const std::vector<const Variant*>& vars, GroupHost& gh) {
+// Takes a planned screen into the group.
+void adopt_screen(PatternGroup& g, const ScreenPlan& plan) {
+  g.screen_on = plan.on;
+  g.screen = plan.geom;
+  g.screen_level = plan.level;
+}
+
+void build_group_host(int kind, PatternGroup& g, const std::vector<const Variant*>& vars, GroupHost& gh) {
   const size_t V = vars.size();
+  if (kind == 0) plan_screen(vars, g.gids, g.L, -1, gh.screen);
+  else gh.screen = ScreenPlan();
+  adopt_screen(g, gh.screen);
+  if (g.screen_on) {
+    g.screen_levels = gh.screen.candidates;
+    g.nonN_sum = 0;
+    for (const Variant* v : vars) g.nonN_sum += (double)(v->key.size() - std::count(v->key.begin(), v->key.end(), 'N'));
+    g.bs_slots = 0;
+    return;
+  }
   const size_t msz = g.nw == 1 ? sizeof(VariantMask<1>) : sizeof(VariantMask<2>);
   gh.masks.assign(std::max<size_t>(V, 1) * msz, 0);
   int maxpos = 0;
@@ -439,7 +456,7 @@ void build_group_host(bool force_popc, PatternGroup& g, const std::vector<const 
     thr[i] = var.threshold;
     npos[i] = (uint32_t)c;
   }
-  g.bs_slots = force_popc ? 0 : bs_slots_for(maxpos);
+  g.bs_slots = kind == 1 ? 0 : bs_slots_for(maxpos);
   g.bs_narrow = g.bs_slots && bs_narrow_ok(g.bs_slots, thr.data(), npos.data(), V);
   gh.prog.clear();
   gh.pgid.clear();
@@ -450,7 +467,21 @@ void build_group_host(bool force_popc, PatternGroup& g, const std::vector<const 
                       &g.bs_candidates);
 }
 
+// Copies a planned screen's records and fills its tables on `st`.
+cof_status upload_screen(cof_handle* h, const ScreenPlan& plan, int nw, DevBuf& records, DevBuf& first, DevBuf& tables,
+                         cudaStream_t st) {
+  COF_CUDA(h, records.ensure(plan.records.size() * 4));
+  COF_CUDA(h, first.ensure(plan.first.size() * 4));
+  COF_CUDA(h, tables.ensure((size_t)plan.geom.words * plan.geom.entries * 4));
+  COF_CUDA(h, cudaMemcpyAsync(records.p, plan.records.data(), plan.records.size() * 4, cudaMemcpyHostToDevice, st));
+  COF_CUDA(h, cudaMemcpyAsync(first.p, plan.first.data(), plan.first.size() * 4, cudaMemcpyHostToDevice, st));
+  launch_screen_tables(plan.geom, nw, records.as<uint32_t>(), first.as<uint32_t>(), tables.as<uint32_t>(), st);
+  COF_CUDA(h, cudaGetLastError());
+  return COF_OK;
+}
+
 cof_status upload_group(cof_handle* h, PatternGroup& g, const GroupHost& gh, cudaStream_t st) {
+  if (g.screen_on) return upload_screen(h, gh.screen, g.nw, g.screen_records, g.screen_first, g.screen_tables, st);
   COF_CUDA(h, g.vmask.ensure(gh.masks.size()));
   COF_CUDA(h, cudaMemcpyAsync(g.vmask.p, gh.masks.data(), gh.masks.size(), cudaMemcpyHostToDevice, st));
   if (g.bs_slots) {
@@ -464,12 +495,28 @@ cof_status upload_group(cof_handle* h, PatternGroup& g, const GroupHost& gh, cud
 
 cof_status build_group_tables(cof_handle* h, PatternGroup& g, const std::vector<const Variant*>& vars) {
   GroupHost gh;
-  build_group_host(h->force_popc, g, vars, gh);
+  build_group_host(h->comparer_kind, g, vars, gh);
   cof_status st = upload_group(h, g, gh, h->stream);
   if (st) return st;
   // The host vectors die on return: wait for the copies.
   COF_CUDA(h, cudaStreamSynchronize(h->stream));
   return COF_OK;
+}
+
+void launch_group_compare(const GenomeView& gv, const PatternGroup& g, const uint32_t* q, const uint32_t* qc,
+                          uint32_t* tile_ctr, uint64_t pos0, uint64_t* hits, unsigned long long* hit_count,
+                          uint64_t hit_cap, int sm_count, cudaStream_t stream) {
+  if (g.screen_on) {
+    launch_screen(gv, q, qc, pos0, g.screen, g.nw, g.screen_records.as<uint32_t>(), g.screen_first.as<uint32_t>(),
+                  g.screen_tables.as<uint32_t>(), g.L, hits, hit_count, hit_cap, sm_count, stream);
+    return;
+  }
+  if (!g.bs_slots ||
+      !launch_comparer_bs(gv, q, qc, pos0, g.bs_prog.as<uint32_t>(), g.bs_pgid.as<uint32_t>(), g.bs_chunks, g.bs_m,
+                          g.bs_slots, g.bs_narrow, g.L, g.concrete_only, tile_ctr, hits, hit_count, hit_cap, sm_count,
+                          stream))
+    launch_comparer(gv, q, qc, pos0, g.vmask.p, (uint32_t)g.gids.size(), g.nw, g.L, hits, hit_count, hit_cap, sm_count,
+                    stream);
 }
 
 void append_format_tables(const Job& job, std::vector<VariantFmt>& vf, std::vector<ShapeFmt>& sf, std::string& pool) {
@@ -519,7 +566,8 @@ using namespace cof::eng;
 // model's choice.
 cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<const Variant*>& vars) {
   g.bs_tuned.clear();
-  if (!g.bs_slots || g.bs_candidates.size() < 2) return COF_OK;
+  g.screen_tuned.clear();
+  if (g.screen_on ? g.screen_levels.size() < 2 : !g.bs_slots || g.bs_candidates.size() < 2) return COF_OK;
   const DevGenome& dg = h->genome;
   const uint64_t npos = dg.n >= g.L ? dg.n - g.L + 1 : 0;
   const uint64_t words = (npos + 31) / 32;
@@ -537,8 +585,55 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
   launch_finder(gv, w0, w1, g.fpat, q, qc, h->stream);
   cudaEvent_t ev[2] = {nullptr, nullptr};
   for (cudaEvent_t& e : ev) COF_CUDA(h, cudaEventCreate(&e));
-  const uint32_t row = (uint32_t)bs_row_for(g.L);
   float best_us = 1e30f;
+  if (g.screen_on) {
+    // The screen's partitions, each timed with tables of its own.
+    ScreenPlan best_plan;
+    DevBuf best_buf[3];
+    cof_status ts = COF_OK;
+    for (uint32_t level : g.screen_levels) {
+      ScreenPlan plan;
+      plan_screen(vars, g.gids, g.L, (int)level, plan);
+      if (!plan.on) continue;
+      DevBuf buf[3];
+      float us = 1e30f;
+      auto run = [&]() -> cof_status {
+        cof_status st = upload_screen(h, plan, g.nw, buf[0], buf[1], buf[2], h->stream);
+        if (st) return st;
+        for (int rep = 0; rep < 2; ++rep) {
+          COF_CUDA(h, cudaMemsetAsync(h->hit_count.p, 0, 8, h->stream));
+          COF_CUDA(h, cudaEventRecord(ev[0], h->stream));
+          launch_screen(gv, q, qc, w0 * 32, plan.geom, g.nw, buf[0].as<uint32_t>(), buf[1].as<uint32_t>(),
+                        buf[2].as<uint32_t>(), g.L, h->hits.as<uint64_t>(), h->hit_count.as<unsigned long long>(), cap,
+                        h->sm_count, h->stream);
+          COF_CUDA(h, cudaEventRecord(ev[1], h->stream));
+          COF_CUDA(h, cudaEventSynchronize(ev[1]));
+          float ms = 0;
+          COF_CUDA(h, cudaEventElapsedTime(&ms, ev[0], ev[1]));
+          us = std::min(us, ms * 1e3f);
+        }
+        COF_CUDA(h, cudaGetLastError());
+        return COF_OK;
+      };
+      if ((ts = run())) break;
+      g.screen_tuned.emplace_back(level, us);
+      if (us < best_us) {
+        best_us = us;
+        best_plan = std::move(plan);
+        for (int i = 0; i < 3; ++i) best_buf[i] = std::move(buf[i]);
+      }
+    }
+    for (cudaEvent_t e : ev) cudaEventDestroy(e);
+    if (ts) return ts;
+    if (best_plan.on && best_plan.level != g.screen_level) {
+      adopt_screen(g, best_plan);
+      g.screen_records = std::move(best_buf[0]);
+      g.screen_first = std::move(best_buf[1]);
+      g.screen_tables = std::move(best_buf[2]);
+    }
+    return COF_OK;
+  }
+  const uint32_t row = (uint32_t)bs_row_for(g.L);
   uint32_t best_m = g.bs_m, best_chunks = g.bs_chunks;
   std::vector<uint32_t> best_prog, best_pgid;
   cof_status st = COF_OK;
@@ -770,14 +865,8 @@ cof_status run_passes(cof_handle* h, uint64_t hit_cap, std::vector<EventPair>& e
       COF_CUDA(h, cudaStreamWaitEvent(h->stream, h->ev_found[b], 0));
       // Comparer units are filled in from qcounts after the search.
       if ((st = record_start(h, evs, "comparer", (double)(s * G + gi), h->stream))) return st;
-      const uint32_t V = (uint32_t)g.gids.size();
-      if (!g.bs_slots ||
-          !launch_comparer_bs(gv, q, qc, w0 * 32, g.bs_prog.as<uint32_t>(), g.bs_pgid.as<uint32_t>(),
-                              g.bs_chunks, g.bs_m, g.bs_slots, g.bs_narrow, g.L, g.concrete_only, qc + nq,
-                              h->hits.as<uint64_t>(), h->hit_count.as<unsigned long long>(), hit_cap, h->sm_count,
-                              h->stream))
-        launch_comparer(gv, q, qc, w0 * 32, g.vmask.p, V, g.nw, g.L, h->hits.as<uint64_t>(),
-                        h->hit_count.as<unsigned long long>(), hit_cap, h->sm_count, h->stream);
+      launch_group_compare(gv, g, q, qc, qc + nq, w0 * 32, h->hits.as<uint64_t>(),
+                           h->hit_count.as<unsigned long long>(), hit_cap, h->sm_count, h->stream);
       if ((st = record_stop(h, evs, h->stream))) return st;
       COF_CUDA(h, cudaEventRecord(h->ev_used[b], h->stream));
       ++pass;
@@ -821,7 +910,10 @@ std::string pass_graph_key(const cof_handle* h, uint64_t cap) {
     for (uint64_t v : {(uint64_t)g.L, (uint64_t)g.nw, (uint64_t)g.bs_slots, (uint64_t)g.bs_narrow, (uint64_t)g.bs_chunks, (uint64_t)g.bs_m,
                        (uint64_t)g.concrete_only, (uint64_t)g.gids.size()})
       put64(v);
-    for (const void* p : {g.bs_prog.p, g.bs_pgid.p, g.vmask.p}) put64((uint64_t)p);
+    for (const void* p : {g.bs_prog.p, g.bs_pgid.p, g.vmask.p, g.screen_records.p, g.screen_first.p, g.screen_tables.p})
+      put64((uint64_t)p);
+    put64(g.screen_on);
+    put(&g.screen, sizeof(g.screen));
     put(&g.fpat, sizeof(g.fpat));
   }
   return k;
@@ -1598,6 +1690,34 @@ int cofx_bs_programs(const char* input, size_t len, uint32_t* info, uint32_t* pr
   return 0;
 }
 
+int cofx_screen_plan(const char* input, size_t len, int level, uint32_t* info, uint32_t* records, size_t records_cap,
+                     uint32_t* first, size_t first_cap) {
+  Job job;
+  std::string err;
+  if (!input || !info || !parse_job(input, len, job, err)) return 1;
+  std::vector<const Variant*> vars;
+  std::vector<uint32_t> gids;
+  for (size_t v = 0; v < job.variants.size(); ++v) {
+    vars.push_back(&job.variants[v]);
+    gids.push_back((uint32_t)v);
+  }
+  const uint32_t L = (uint32_t)job.pattern.size();
+  ScreenPlan plan;
+  plan_screen(vars, gids, L, level, plan);
+  const ScreenGeom& G = plan.geom;
+  uint32_t* o = info;
+  for (uint32_t x : {(uint32_t)plan.on, L, G.K}) *o++ = x;
+  for (const uint32_t* a : {G.a, G.q, G.base, G.cap})
+    for (int k = 0; k < kScreenRuns; ++k) *o++ = a[k];
+  for (uint32_t x : {G.entries, G.bits, G.fields, G.top, G.words, G.degenerate, (uint32_t)vars.size(),
+                     screen_record_words(L <= 32 ? 1 : 2)})
+    *o++ = x;
+  if (records && records_cap >= plan.records.size())
+    std::copy(plan.records.begin(), plan.records.end(), records);
+  if (first && first_cap >= plan.first.size()) std::copy(plan.first.begin(), plan.first.end(), first);
+  return 0;
+}
+
 void cofx_mismatch_table(uint8_t* out) {
   if (!out) return;
   for (int p = 0; p < 256; ++p)
@@ -1626,7 +1746,7 @@ uint64_t cof_pack_text(const char* seq, uint64_t n, uint32_t* hi, uint32_t* lo, 
 
 cof_status cof_set_comparer(cof_handle* h, int kind) {
   if (!h || kind < 0 || kind > 2) return COF_ERR_ARG;
-  h->force_popc = kind == 1;
+  h->comparer_kind = kind;
   h->jobs_on_device = false;  // rebuild the comparer tables on the next search
   return COF_OK;
 }
@@ -1645,7 +1765,18 @@ cof_status cof_schedule_text(cof_handle* h, const char** text, size_t* len) {
     char line[256];
     snprintf(line, sizeof line, "%s variants=%zu slots=%d", g.pattern.c_str(), g.gids.size(), g.bs_slots);
     t += line;
-    if (g.bs_slots) {
+    if (g.screen_on) {
+      snprintf(line, sizeof line, " screen %s words=%u runs=%u", screen_level_name(g.screen_level), g.screen.words,
+               g.screen.K);
+      t += line;
+      if (!g.screen_tuned.empty()) {
+        t += " tuned:";
+        for (const auto& x : g.screen_tuned) {
+          snprintf(line, sizeof line, " [%s %.1fus]", screen_level_name(x.first), x.second);
+          t += line;
+        }
+      }
+    } else if (g.bs_slots) {
       snprintf(line, sizeof line, " m=%u chunks=%u planes=%s", g.bs_m, g.bs_chunks,
                g.bs_narrow && g.bs_m > 1 ? "NB" : "NB+1");
       t += line;
@@ -1671,7 +1802,7 @@ cof_status cof_comparer_info(const cof_handle* h, int* kind, int* slots) {
   if (!h) return COF_ERR_ARG;
   int k = 0, sl = 0;
   for (const PatternGroup& g : h->groups) {
-    k = std::max(k, g.bs_slots ? 2 : 1);
+    k = std::max(k, g.screen_on ? 3 : g.bs_slots ? 2 : 1);
     sl = std::max(sl, g.bs_slots);
   }
   if (kind) *kind = k ? k : 1;

@@ -13,6 +13,7 @@
 #include "../../include/cof.h"
 #include "cof_internal.h"
 #include "kernels.cuh"
+#include "screen.cuh"
 
 namespace cof {
 namespace eng {
@@ -124,6 +125,13 @@ struct PatternGroup {
   std::vector<uint32_t> bs_candidates;             // lengths m worth timing (cost model's best first)
   std::vector<std::pair<uint32_t, float>> bs_tuned;  // (m, comparer µs per segment) measured by the autotuner
   DevBuf vmask, bs_prog, bs_pgid;
+  // Table screen (screen.cuh); where it runs, bs_slots is 0.
+  bool screen_on = false;
+  ScreenGeom screen;
+  uint32_t screen_level = 0;
+  std::vector<uint32_t> screen_levels;                  // partitions worth timing (cost model's best first)
+  std::vector<std::pair<uint32_t, float>> screen_tuned;  // (partition, µs per segment) measured by the autotuner
+  DevBuf screen_records, screen_first, screen_tables;
 };
 
 }  // namespace eng
@@ -158,7 +166,7 @@ struct cof_handle {
   std::vector<Job> jobs;
   std::vector<uint32_t> job_gid0;
   bool jobs_on_device = false;
-  bool force_popc = false;
+  int comparer_kind = 0;  // cof_set_comparer
   std::vector<PatternGroup> groups;  // jobs sharing a padded pattern share finder + comparer passes
   DevBuf vfmt, sfmt, pool;           // row formatting tables over all variants
   DevGenome genome, scratch;
@@ -223,14 +231,22 @@ void pinned_release(cof_handle* h, void* p, size_t cap);
 struct GroupHost {
   std::vector<unsigned char> masks;  // popcount comparer (only when the bit-sliced one cannot run)
   std::vector<uint32_t> prog, pgid;  // bit-sliced lane programs
+  ScreenPlan screen;                 // table screen (then the others stay empty)
 };
-// Fills g's host-side fields (slots, chunks, m, ...) and `gh` for `vars`
-// (ids g.gids).  Thread-safe: touches only its arguments.
-void build_group_host(bool force_popc, PatternGroup& g, const std::vector<const Variant*>& vars, GroupHost& gh);
+// Fills g's host-side fields (slots, chunks, m, screen, ...) and `gh` for
+// `vars` (ids g.gids); `kind` as cof_set_comparer.  Thread-safe: touches only
+// its arguments.
+void build_group_host(int kind, PatternGroup& g, const std::vector<const Variant*>& vars, GroupHost& gh);
 // Copies `gh` into g's device buffers on `st`; gh must stay alive until the
 // copies are done.
 cof_status upload_group(cof_handle* h, PatternGroup& g, const GroupHost& gh, cudaStream_t st);
 cof_status build_group_tables(cof_handle* h, PatternGroup& g, const std::vector<const Variant*>& vars);
+// Compares the candidates of one finder pass (queue `q`, count `qc`, segment
+// starting at `pos0`) with g's variants: screen, bit-sliced or popcount
+// comparer.  `tile_ctr`: a zeroed u32 of this launch.
+void launch_group_compare(const GenomeView& gv, const PatternGroup& g, const uint32_t* q, const uint32_t* qc,
+                          uint32_t* tile_ctr, uint64_t pos0, uint64_t* hits, unsigned long long* hit_count,
+                          uint64_t hit_cap, int sm_count, cudaStream_t stream);
 // Lane programs of the bit-sliced comparer for `vars` (ids `gids`), `S` slots,
 // class rows of `row` words; layout in kernels.cuh.
 // force_m (1-24) replaces the cost model's choice of m; `ranked` (may be

@@ -180,7 +180,7 @@ void builder_main(cof_server* s) {
     }
     ts->host.resize(ts->groups.size());
     for (size_t g = 0; g < ts->groups.size(); ++g)
-      build_group_host(s->h->force_popc, ts->groups[g], vars[g], ts->host[g]);
+      build_group_host(s->h->comparer_kind, ts->groups[g], vars[g], ts->host[g]);
     {
       std::lock_guard<std::mutex> lock(s->mu);
       s->built = std::move(ts);
@@ -273,14 +273,8 @@ cof_status run_step(cof_server* s, uint64_t k) {
       launch_finder(gv, w0, w1, g.fpat, q, qc, h->stream2);
       COF_CUDA(h, cudaEventRecord(h->ev_found[b], h->stream2));
       COF_CUDA(h, cudaStreamWaitEvent(h->stream, h->ev_found[b], 0));
-      const uint32_t V = (uint32_t)g.gids.size();
-      if (!g.bs_slots ||
-          !launch_comparer_bs(gv, q, qc, w0 * 32, g.bs_prog.as<uint32_t>(), g.bs_pgid.as<uint32_t>(),
-                              g.bs_chunks, g.bs_m, g.bs_slots, g.bs_narrow, g.L, g.concrete_only, qc + nq,
-                              s->step_hits.as<uint64_t>(), s->step_count.as<unsigned long long>(), cap, h->sm_count,
-                              h->stream))
-        launch_comparer(gv, q, qc, w0 * 32, g.vmask.p, V, g.nw, g.L, s->step_hits.as<uint64_t>(),
-                        s->step_count.as<unsigned long long>(), cap, h->sm_count, h->stream);
+      launch_group_compare(gv, g, q, qc, qc + nq, w0 * 32, s->step_hits.as<uint64_t>(),
+                           s->step_count.as<unsigned long long>(), cap, h->sm_count, h->stream);
       COF_CUDA(h, cudaEventRecord(h->ev_used[b], h->stream));
       ++pass;
     }
@@ -572,6 +566,7 @@ void worker_main(cof_server* s) {
       for (size_t g = 0; g < fresh->groups.size() && !st; ++g) {
         PatternGroup& pg = fresh->groups[g];
         pg.vmask.st = pg.bs_prog.st = pg.bs_pgid.st = h->stream;
+        pg.screen_records.st = pg.screen_first.st = pg.screen_tables.st = h->stream;
         st = upload_group(h, pg, fresh->host[g], h->stream);
       }
       s->tables = std::move(fresh);

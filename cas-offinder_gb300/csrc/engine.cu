@@ -421,11 +421,12 @@ void adopt_screen(PatternGroup& g, const ScreenPlan& plan) {
   g.screen_on = plan.on;
   g.screen = plan.geom;
   g.screen_level = plan.level;
+  g.screen_scans = plan.on && plan.scans;
 }
 
 void build_group_host(int kind, PatternGroup& g, const std::vector<const Variant*>& vars, GroupHost& gh) {
   const size_t V = vars.size();
-  if (kind == 0) plan_screen(vars, g.gids, g.L, -1, gh.screen);
+  if (kind == 0) plan_screen(vars, g.gids, g.fpat, -1, gh.screen);
   else gh.screen = ScreenPlan();
   adopt_screen(g, gh.screen);
   if (g.screen_on) {
@@ -472,7 +473,7 @@ cof_status upload_screen(cof_handle* h, const ScreenPlan& plan, int nw, DevBuf& 
                          cudaStream_t st) {
   COF_CUDA(h, records.ensure(plan.records.size() * 4));
   COF_CUDA(h, first.ensure(plan.first.size() * 4));
-  COF_CUDA(h, tables.ensure((size_t)plan.geom.words * plan.geom.entries * 4));
+  COF_CUDA(h, tables.ensure((size_t)plan.geom.words * screen_entries(plan.geom.K) * 4));
   COF_CUDA(h, cudaMemcpyAsync(records.p, plan.records.data(), plan.records.size() * 4, cudaMemcpyHostToDevice, st));
   COF_CUDA(h, cudaMemcpyAsync(first.p, plan.first.data(), plan.first.size() * 4, cudaMemcpyHostToDevice, st));
   launch_screen_tables(plan.geom, nw, records.as<uint32_t>(), first.as<uint32_t>(), tables.as<uint32_t>(), st);
@@ -503,20 +504,44 @@ cof_status build_group_tables(cof_handle* h, PatternGroup& g, const std::vector<
   return COF_OK;
 }
 
-void launch_group_compare(const GenomeView& gv, const PatternGroup& g, const uint32_t* q, const uint32_t* qc,
-                          uint32_t* tile_ctr, uint64_t pos0, uint64_t* hits, unsigned long long* hit_count,
-                          uint64_t hit_cap, int sm_count, cudaStream_t stream) {
+namespace {
+ScreenList screen_list(const cof_handle* h) {
+  ScreenList l;
+  l.items = h->screen_items.as<uint4>();
+  l.counts = h->screen_counts.as<uint32_t>();
+  l.room = h->screen_items.cap / sizeof(uint4);
+  return l;
+}
+}  // namespace
+
+cof_status ensure_screen_list(cof_handle* h, uint64_t positions) {
+  COF_CUDA(h, h->screen_items.ensure(screen_list_items(positions) * sizeof(uint4)));
+  COF_CUDA(h, h->screen_counts.ensure(screen_lists(h->sm_count) * 4));
+  return COF_OK;
+}
+
+void launch_group_compare(const cof_handle* h, const PatternGroup& g, const uint32_t* q, const uint32_t* qc,
+                          uint32_t* tile_ctr, uint64_t pos0, const HitSink& sink) {
+  const GenomeView gv = h->genome.view();
   if (g.screen_on) {
-    launch_screen(gv, q, qc, pos0, g.screen, g.nw, g.screen_records.as<uint32_t>(), g.screen_first.as<uint32_t>(),
-                  g.screen_tables.as<uint32_t>(), g.L, hits, hit_count, hit_cap, sm_count, stream);
+    launch_screen(gv, q, qc, pos0, g.screen, g.nw, g.screen_tb(), g.L, screen_list(h), sink, h->sm_count, h->stream);
     return;
   }
   if (!g.bs_slots ||
       !launch_comparer_bs(gv, q, qc, pos0, g.bs_prog.as<uint32_t>(), g.bs_pgid.as<uint32_t>(), g.bs_chunks, g.bs_m,
-                          g.bs_slots, g.bs_narrow, g.L, g.concrete_only, tile_ctr, hits, hit_count, hit_cap, sm_count,
-                          stream))
-    launch_comparer(gv, q, qc, pos0, g.vmask.p, (uint32_t)g.gids.size(), g.nw, g.L, hits, hit_count, hit_cap, sm_count,
-                    stream);
+                          g.bs_slots, g.bs_narrow, g.L, g.concrete_only, tile_ctr, sink.hits, sink.count, sink.cap,
+                          h->sm_count, h->stream))
+    launch_comparer(gv, q, qc, pos0, g.vmask.p, (uint32_t)g.gids.size(), g.nw, g.L, sink.hits, sink.count, sink.cap,
+                    h->sm_count, h->stream);
+}
+
+void launch_group_scan(const cof_handle* h, const PatternGroup& g, uint64_t w0, uint64_t w1, uint32_t* qc,
+                       const HitSink& sink) {
+  // Equal pieces of at most kScanWords.
+  const uint64_t pieces = (w1 - w0 + kScanWords - 1) / kScanWords;
+  for (uint64_t i = 0; i < pieces; ++i)
+    launch_scan_screen(h->genome.view(), w0 + (w1 - w0) * i / pieces, w0 + (w1 - w0) * (i + 1) / pieces, g.fpat,
+                       g.screen, g.screen_tb(), screen_list(h), qc, sink, h->sm_count, h->stream);
 }
 
 void append_format_tables(const Job& job, std::vector<VariantFmt>& vf, std::vector<ShapeFmt>& sf, std::string& pool) {
@@ -573,7 +598,11 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
   const uint64_t words = (npos + 31) / 32;
   if (words < 2 * kSegWords) return COF_OK;
   const uint64_t w0 = (words / kSegWords / 2) * kSegWords, w1 = std::min(words, w0 + kSegWords);
-  COF_CUDA(h, h->queue[0].ensure(2 * kSegPositions * 4));
+  if (!g.screen_scans || g.screen_levels.size() > 1) COF_CUDA(h, h->queue[0].ensure(2 * kSegPositions * 4));
+  if (g.screen_on) {
+    cof_status st = ensure_screen_list(h, std::min<uint64_t>(dg.n, 32 * kScanWords));
+    if (st) return st;
+  }
   COF_CUDA(h, h->qcounts.ensure(std::max<size_t>(h->qcounts.cap, 8)));  // count, tile counter
   COF_CUDA(h, h->hit_count.ensure(8));
   const uint64_t cap = std::max<uint64_t>(h->hits.cap / 8, 1u << 20);
@@ -582,7 +611,7 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
   uint32_t* q = h->queue[0].as<uint32_t>();
   uint32_t* qc = h->qcounts.as<uint32_t>();
   COF_CUDA(h, cudaMemsetAsync(qc, 0, 4, h->stream));
-  launch_finder(gv, w0, w1, g.fpat, q, qc, h->stream);
+  if (!g.screen_on) launch_finder(gv, w0, w1, g.fpat, q, qc, h->stream);
   cudaEvent_t ev[2] = {nullptr, nullptr};
   for (cudaEvent_t& e : ev) COF_CUDA(h, cudaEventCreate(&e));
   float best_us = 1e30f;
@@ -593,7 +622,7 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
     cof_status ts = COF_OK;
     for (uint32_t level : g.screen_levels) {
       ScreenPlan plan;
-      plan_screen(vars, g.gids, g.L, (int)level, plan);
+      plan_screen(vars, g.gids, g.fpat, (int)level, plan);
       if (!plan.on) continue;
       DevBuf buf[3];
       float us = 1e30f;
@@ -602,10 +631,16 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
         if (st) return st;
         for (int rep = 0; rep < 2; ++rep) {
           COF_CUDA(h, cudaMemsetAsync(h->hit_count.p, 0, 8, h->stream));
+          COF_CUDA(h, cudaMemsetAsync(qc, 0, 4, h->stream));
           COF_CUDA(h, cudaEventRecord(ev[0], h->stream));
-          launch_screen(gv, q, qc, w0 * 32, plan.geom, g.nw, buf[0].as<uint32_t>(), buf[1].as<uint32_t>(),
-                        buf[2].as<uint32_t>(), g.L, h->hits.as<uint64_t>(), h->hit_count.as<unsigned long long>(), cap,
-                        h->sm_count, h->stream);
+          const ScreenTables tb{buf[0].as<uint32_t>(), buf[1].as<uint32_t>(), buf[2].as<uint32_t>()};
+          const HitSink sink{h->hits.as<uint64_t>(), h->hit_count.as<unsigned long long>(), cap};
+          if (plan.scans) {
+            launch_scan_screen(gv, w0, w1, g.fpat, plan.geom, tb, screen_list(h), qc, sink, h->sm_count, h->stream);
+          } else {
+            launch_finder(gv, w0, w1, g.fpat, q, qc, h->stream);
+            launch_screen(gv, q, qc, w0 * 32, plan.geom, g.nw, tb, g.L, screen_list(h), sink, h->sm_count, h->stream);
+          }
           COF_CUDA(h, cudaEventRecord(ev[1], h->stream));
           COF_CUDA(h, cudaEventSynchronize(ev[1]));
           float ms = 0;
@@ -831,14 +866,38 @@ cof_status run_passes(cof_handle* h, uint64_t hit_cap, std::vector<EventPair>& e
     cof_status st = queue_upload_ahead(h);
     if (st) return st;
   }
+  const HitSink sink{h->hits.as<uint64_t>(), h->hit_count.as<unsigned long long>(), hit_cap};
   uint64_t pass = 0;
   for (uint64_t s = 0; s < nseg; ++s) {
+    bool waited = false;  // h->stream has the planes of segment s of a streamed upload
     for (size_t gi = 0; gi < G; ++gi) {
       const PatternGroup& g = h->groups[gi];
       const uint64_t npos = dg.n >= g.L ? dg.n - g.L + 1 : 0;
       const uint64_t words = (npos + 31) / 32;
       const uint64_t w0 = s * kSegWords, w1 = std::min(words, w0 + kSegWords);
       if (w0 >= w1 || g.gids.empty()) continue;
+      if (g.screen_scans) {
+        // The whole genome at once; during a streamed upload, segment by
+        // segment as the planes arrive.
+        if (s > 0 && !h->upload_pending) continue;
+        if (h->upload_pending && !waited) {
+          if (ahead) {
+            COF_CUDA(h, cudaStreamWaitEvent(h->stream, h->upload_ev[std::min<size_t>(s, h->upload_pending - 1)], 0));
+          } else {
+            cof_status st = issue_upload(h, (size_t)s + 2);
+            if (st) return st;
+            COF_CUDA(h, cudaEventRecord(h->ev_start, h->stream2));
+            COF_CUDA(h, cudaStreamWaitEvent(h->stream, h->ev_start, 0));
+          }
+          waited = true;
+        }
+        uint32_t* qc = h->qcounts.as<uint32_t>() + s * G + gi;
+        cof_status st = record_start(h, evs, "comparer", (double)(s * G + gi), h->stream);
+        if (st) return st;
+        launch_group_scan(h, g, w0, h->upload_pending ? w1 : words, qc, sink);
+        if ((st = record_stop(h, evs, h->stream))) return st;
+        continue;
+      }
       const int b = (int)(pass & 1);
       uint32_t* qc = h->qcounts.as<uint32_t>() + s * G + gi;
       uint32_t* q = h->queue[b].as<uint32_t>();
@@ -865,8 +924,7 @@ cof_status run_passes(cof_handle* h, uint64_t hit_cap, std::vector<EventPair>& e
       COF_CUDA(h, cudaStreamWaitEvent(h->stream, h->ev_found[b], 0));
       // Comparer units are filled in from qcounts after the search.
       if ((st = record_start(h, evs, "comparer", (double)(s * G + gi), h->stream))) return st;
-      launch_group_compare(gv, g, q, qc, qc + nq, w0 * 32, h->hits.as<uint64_t>(),
-                           h->hit_count.as<unsigned long long>(), hit_cap, h->sm_count, h->stream);
+      launch_group_compare(h, g, q, qc, qc + nq, w0 * 32, sink);
       if ((st = record_stop(h, evs, h->stream))) return st;
       COF_CUDA(h, cudaEventRecord(h->ev_used[b], h->stream));
       ++pass;
@@ -900,6 +958,8 @@ std::string pass_graph_key(const cof_handle* h, uint64_t cap) {
     put64((uint64_t)p);
   put64(h->genome.n);
   put64(h->qcounts.cap);
+  for (const void* p : {h->screen_items.p, h->screen_counts.p}) put64((uint64_t)p);
+  put64(h->screen_items.cap);
   // A streamed upload's copies are part of the graph.
   put64(h->upload_pending);
   for (const uint32_t* p : h->upload_src) put64(h->upload_pending ? (uint64_t)p : 0);
@@ -913,6 +973,7 @@ std::string pass_graph_key(const cof_handle* h, uint64_t cap) {
     for (const void* p : {g.bs_prog.p, g.bs_pgid.p, g.vmask.p, g.screen_records.p, g.screen_first.p, g.screen_tables.p})
       put64((uint64_t)p);
     put64(g.screen_on);
+    put64(g.screen_scans);
     put(&g.screen, sizeof(g.screen));
     put(&g.fpat, sizeof(g.fpat));
   }
@@ -1018,8 +1079,14 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
   h->job_byte0.assign(J + 1, 0);
   if (h->summaries.size() != J) h->summaries.assign(J, {});
   if (h->job_gid0.back() == 0) return COF_OK;
-  COF_CUDA(h, h->queue[0].ensure(2 * kSegPositions * 4));
-  COF_CUDA(h, h->queue[1].ensure(2 * kSegPositions * 4));
+  bool queues = false, screens = false;
+  for (const PatternGroup& g : h->groups) {
+    queues |= !g.screen_scans;
+    screens |= g.screen_on;
+  }
+  if (queues)
+    for (DevBuf& q : h->queue) COF_CUDA(h, q.ensure(2 * kSegPositions * 4));
+  if (screens && (st = ensure_screen_list(h, std::min<uint64_t>(h->genome.n, 32 * kScanWords)))) return st;
   COF_CUDA(h, h->hit_count.ensure(8));
   uint64_t cap = std::max<uint64_t>(h->hits.cap / 8, 1u << 20);
   COF_CUDA(h, h->hits.ensure(cap * 8));
@@ -1702,14 +1769,17 @@ int cofx_screen_plan(const char* input, size_t len, int level, uint32_t* info, u
     gids.push_back((uint32_t)v);
   }
   const uint32_t L = (uint32_t)job.pattern.size();
+  FinderPattern pat{};
   ScreenPlan plan;
-  plan_screen(vars, gids, L, level, plan);
+  if (make_finder_pattern(job.pattern, revcomp(job.pattern), pat)) plan_screen(vars, gids, pat, level, plan);
   const ScreenGeom& G = plan.geom;
   uint32_t* o = info;
   for (uint32_t x : {(uint32_t)plan.on, L, G.K}) *o++ = x;
-  for (const uint32_t* a : {G.a, G.q, G.base, G.cap})
-    for (int k = 0; k < kScreenRuns; ++k) *o++ = a[k];
-  for (uint32_t x : {G.entries, G.bits, G.fields, G.top, G.words, G.degenerate, (uint32_t)vars.size(),
+  for (int k = 0; k < kScreenRuns; ++k) *o++ = G.a0 + screen_run_at(k);
+  for (int k = 0; k < kScreenRuns; ++k) *o++ = screen_run_len(G.K, k);
+  for (int k = 0; k < kScreenRuns; ++k) *o++ = screen_base(k);
+  for (int k = 0; k < kScreenRuns; ++k) *o++ = G.cap[k];
+  for (uint32_t x : {screen_entries(G.K), G.bits, G.fields, G.top, G.words, G.degenerate, (uint32_t)vars.size(),
                      screen_record_words(L <= 32 ? 1 : 2)})
     *o++ = x;
   if (records && records_cap >= plan.records.size())
@@ -1766,8 +1836,8 @@ cof_status cof_schedule_text(cof_handle* h, const char** text, size_t* len) {
     snprintf(line, sizeof line, "%s variants=%zu slots=%d", g.pattern.c_str(), g.gids.size(), g.bs_slots);
     t += line;
     if (g.screen_on) {
-      snprintf(line, sizeof line, " screen %s words=%u runs=%u", screen_level_name(g.screen_level), g.screen.words,
-               g.screen.K);
+      snprintf(line, sizeof line, " screen%s %s words=%u runs=%u", g.screen_scans ? " scanning" : "",
+               screen_level_name(g.screen_level), g.screen.words, g.screen.K);
       t += line;
       if (!g.screen_tuned.empty()) {
         t += " tuned:";

@@ -132,6 +132,10 @@ struct PatternGroup {
   std::vector<uint32_t> screen_levels;                  // partitions worth timing (cost model's best first)
   std::vector<std::pair<uint32_t, float>> screen_tuned;  // (partition, µs per segment) measured by the autotuner
   DevBuf screen_records, screen_first, screen_tables;
+  bool screen_scans = false;  // the screen scans the planes itself: no finder pass, no candidate queue
+  ScreenTables screen_tb() const {
+    return ScreenTables{screen_records.as<uint32_t>(), screen_first.as<uint32_t>(), screen_tables.as<uint32_t>()};
+  }
 };
 
 }  // namespace eng
@@ -171,6 +175,7 @@ struct cof_handle {
   DevBuf vfmt, sfmt, pool;           // row formatting tables over all variants
   DevGenome genome, scratch;
 
+  DevBuf screen_items, screen_counts;  // candidates that passed a screen (ScreenList), used on `stream`
   DevBuf queue[2], qcounts, hits, hits_sorted, summary_counts, hit_count, sort_tmp, row_bytes, row_offsets, row_count, text, small,
       job_start, job_bytes;
   HostPinned host_text;
@@ -243,10 +248,15 @@ cof_status upload_group(cof_handle* h, PatternGroup& g, const GroupHost& gh, cud
 cof_status build_group_tables(cof_handle* h, PatternGroup& g, const std::vector<const Variant*>& vars);
 // Compares the candidates of one finder pass (queue `q`, count `qc`, segment
 // starting at `pos0`) with g's variants: screen, bit-sliced or popcount
-// comparer.  `tile_ctr`: a zeroed u32 of this launch.
-void launch_group_compare(const GenomeView& gv, const PatternGroup& g, const uint32_t* q, const uint32_t* qc,
-                          uint32_t* tile_ctr, uint64_t pos0, uint64_t* hits, unsigned long long* hit_count,
-                          uint64_t hit_cap, int sm_count, cudaStream_t stream);
+// comparer.  `tile_ctr`: a zeroed u32 of this launch.  Runs on h->stream.
+void launch_group_compare(const cof_handle* h, const PatternGroup& g, const uint32_t* q, const uint32_t* qc,
+                          uint32_t* tile_ctr, uint64_t pos0, const HitSink& sink);
+// Scans plane words [w0, w1) for g (screen_scans) on h->stream; candidates
+// are added to *qc.
+void launch_group_scan(const cof_handle* h, const PatternGroup& g, uint64_t w0, uint64_t w1, uint32_t* qc,
+                       const HitSink& sink);
+// The list buffers of the screens of launches over up to `positions` starts.
+cof_status ensure_screen_list(cof_handle* h, uint64_t positions);
 // Lane programs of the bit-sliced comparer for `vars` (ids `gids`), `S` slots,
 // class rows of `row` words; layout in kernels.cuh.
 // force_m (1-24) replaces the cost model's choice of m; `ranked` (may be

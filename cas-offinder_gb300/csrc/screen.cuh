@@ -2,7 +2,7 @@
 // candidate window up in tables of least mismatch counts, and counting only
 // the candidates that the tables cannot rule out.
 //
-// A screen splits (part of) the window into K disjoint runs of at most 7
+// A screen splits (part of) the window into K disjoint runs of 6 or 7
 // positions.  For a class of compare variants, table k holds for each of the
 // 4^q words that run k of a window can spell the least mismatch count of any
 // variant of the class on that run.  The sum over the runs is a lower bound
@@ -28,19 +28,24 @@
 
 namespace cof {
 
-constexpr int kScreenRuns = 4;       // most runs of a screen
-constexpr int kScreenRunMax = 7;     // positions per run at most (4^7 entries of 4 bytes = 64 KiB)
+// Runs of a screen, from its first position `a0` on: three of 7 positions, or
+// four of 7, 7, 6 and 6.  The layout is fixed so that a run's bits are reached
+// by immediate shifts and masks; positions past the window or outside the
+// variants' span mismatch nobody.
+constexpr int kScreenRuns = 4;
+constexpr uint32_t screen_run_at(uint32_t k) { return k < 3 ? 7u * k : 20u; }
+constexpr uint32_t screen_run_len(uint32_t K, uint32_t k) { return K == 4 && k >= 2 ? 6u : 7u; }
+// First entry of each run's table within a word's tables, and their size.
+constexpr uint32_t screen_base(uint32_t k) { return k == 0 ? 0u : k == 1 ? 16384u : k == 2 ? 32768u : 36864u; }
+constexpr uint32_t screen_entries(uint32_t K) { return K == 4 ? 40960u : 49152u; }
 constexpr uint32_t kScreenMaxLimit = 15;  // largest mismatch limit (5-bit fields)
-constexpr uint32_t kScreenMaxWords = 2048;
+constexpr uint32_t kScreenMaxWords = 768;  // a CTA's share spans at most 8 of them
 
 // Geometry of a group's screen (kernel argument).
 struct ScreenGeom {
-  uint32_t K = 0;                // runs (3 or 4)
-  uint32_t a[kScreenRuns] = {};  // first position of each run in the oriented window
-  uint32_t q[kScreenRuns] = {};  // its positions
-  uint32_t base[kScreenRuns] = {};  // first entry of its table within a word's tables
-  uint32_t cap[kScreenRuns] = {};   // largest entry of its table
-  uint32_t entries = 0;          // 32-bit entries of one word's tables
+  uint32_t K = 0;                  // runs (3 or 4)
+  uint32_t a0 = 0;                 // first position of the runs in the oriented window
+  uint32_t cap[kScreenRuns] = {};  // largest entry of each run's table
   uint32_t bits = 4;             // field width F
   uint32_t fields = 8;           // classes per word
   uint32_t top = 0x88888888u;    // the fields' top bits
@@ -55,6 +60,7 @@ constexpr uint32_t screen_record_words(int nw) { return nw == 1 ? 8 : 12; }
 // A planned screen on the host: variants sorted by class.
 struct ScreenPlan {
   bool on = false;
+  bool scans = false;  // the scanning kernel rather than the finder and the screen of its queue
   ScreenGeom geom;
   std::vector<uint32_t> records;  // screen_record_words(nw) per variant
   std::vector<uint32_t> first;    // words * (fields + 1): first record of each class of a word, then the word's end
@@ -62,24 +68,60 @@ struct ScreenPlan {
   std::vector<uint32_t> candidates;  // levels worth timing, the model's best first
 };
 
-// Plans the screen of a pattern group of windows of L positions over `vars`
-// (ids `gids`).  `on` stays false where the screen cannot run (a limit above
+// Plans the screen of a pattern group (PAM scan `pat`) over `vars` (ids
+// `gids`).  `on` stays false where the screen cannot run (a limit above
 // 15) or its cost model puts the bit-sliced comparer ahead.  `force_level`
 // >= 0 takes that partition.
-void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint32_t>& gids, uint32_t L,
+void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint32_t>& gids, const FinderPattern& pat,
                  int force_level, ScreenPlan& plan);
 // Text of a partition ("2/guide", "4 guides", ...).
 const char* screen_level_name(uint32_t level);
 
+// Candidates that passed a class, listed per warp of the screening launch: an
+// item is {position relative to the launch's base << 1 | strand, the passed
+// classes' top bits | kOddWindow | the word relative to the first of its CTA,
+// first word of the oriented window's hi and lo planes}.
+struct ScreenList {
+  uint4* items = nullptr;      // `room` of them, shared out evenly over the warps
+  uint32_t* counts = nullptr;  // items of each warp
+  uint64_t room = 0;
+};
+// Set in an item whose window may hold a non-base byte (a bit that is neither
+// a field's top bit nor part of the relative word).
+constexpr uint32_t kOddWindow = 1u << 5;
+// Most warps of a launch on a device of `sm_count` SMs, and the items
+// `positions` start positions should have room for.  A warp whose list is
+// full counts its further candidates on the spot, so the size only affects
+// the speed.
+uint32_t screen_lists(int sm_count);
+uint64_t screen_list_items(uint64_t positions);
+
+// Device side of a group's screen.
+struct ScreenTables {
+  const uint32_t *records, *first, *tables;
+};
+// Where hits go (as launch_comparer).
+struct HitSink {
+  uint64_t* hits;
+  unsigned long long* count;
+  uint64_t cap;
+};
+
 // Fills the tables of a planned screen from its records (device pointers):
-// geom.words * geom.entries words at `tables`.
+// geom.words * screen_entries(geom.K) words at `tables`.
 void launch_screen_tables(const ScreenGeom& geom, int nw, const uint32_t* records, const uint32_t* first,
                           uint32_t* tables, cudaStream_t stream);
 // Tests every entry of `queue` (count read on the device) against the
 // screen's variants; appends hit keys as launch_comparer does.
 void launch_screen(const GenomeView& g, const uint32_t* queue, const uint32_t* qcount, uint64_t seg_pos0,
-                   const ScreenGeom& geom, int nw, const uint32_t* records, const uint32_t* first,
-                   const uint32_t* tables, uint32_t L, uint64_t* hits, unsigned long long* hit_count,
-                   uint64_t hit_cap, int sm_count, cudaStream_t stream);
+                   const ScreenGeom& geom, int nw, const ScreenTables& tb, uint32_t L, const ScreenList& list,
+                   const HitSink& sink, int sm_count, cudaStream_t stream);
+// PAM scan and screen in one kernel, without a candidate queue, for windows
+// of up to 32 positions: plane words [w_begin, w_end), at most
+// kScanWords of them; adds the candidates found to *qcount.
+constexpr uint64_t kScanWords = 1ull << 24;
+void launch_scan_screen(const GenomeView& g, uint64_t w_begin, uint64_t w_end, const FinderPattern& pat,
+                        const ScreenGeom& geom, const ScreenTables& tb, const ScreenList& list, uint32_t* qcount,
+                        const HitSink& sink, int sm_count, cudaStream_t stream);
 
 }  // namespace cof

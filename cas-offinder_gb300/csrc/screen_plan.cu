@@ -45,10 +45,28 @@ struct Guide {
 
 const char* screen_level_name(uint32_t level) { return level < kLevelCount ? kLevels[level].name : "?"; }
 
-void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint32_t>& gids, uint32_t L,
+namespace {
+
+// Costs in SM clocks per 2,048 starts, of which `c` are candidates (measured
+// at 0.08 and 0.2 candidates per start: 280 and 533 for one scanning word,
+// 227 and 265 for the finder, 0.88 per candidate and word of the queue).
+double scan_cost(double c, double words) { return words * (100.0 + 1.08 * c); }
+double finder_cost(double c) { return 182.0 + 0.22 * c; }
+double queue_cost(double c, double words) { return finder_cost(c) + words * (15.0 + 0.88 * c); }
+
+// The scanning kernel stages up to 320 of 2,048 starts' candidates at a time
+// and takes one-word windows.
+bool can_scan(const FinderPattern& pat, double plus, double minus) {
+  return pat.L <= 32 && std::max(plus, minus) <= 0.14;
+}
+
+}  // namespace
+
+void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint32_t>& gids, const FinderPattern& pat,
                  int force_level, ScreenPlan& plan) {
   plan = ScreenPlan();
   const size_t V = vars.size();
+  const uint32_t L = pat.L;
   if (V == 0 || L == 0 || L > (uint32_t)kMaxL) return;
   uint32_t limit = 0;
   for (const Variant* v : vars) limit = std::max<uint32_t>(limit, v->threshold);
@@ -68,9 +86,9 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
   while (p1 > p0 && !cover[p1 - 1]) --p1;
   const uint32_t span = p1 - p0;
   if (span < 9) return;
-  // Three runs of up to 7 positions for spans up to 23 (192 KiB of tables at
-  // most), four runs of 7, 7, 6, 6 (160 KiB) beyond; of a longer span, the
-  // stretch that the most variants use.
+  // Three runs of 7 positions (192 KiB of tables) for spans up to 23, four
+  // of 7, 7, 6, 6 (160 KiB) beyond; of a longer span, the stretch that the
+  // most variants use.
   G.K = span <= 23 ? 3 : 4;
   const uint32_t take = std::min<uint32_t>(span, G.K == 3 ? 21 : 26);
   uint32_t best_s = p0;
@@ -80,14 +98,7 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
     for (uint32_t k = s; k < s + take; ++k) c += cover[k];
     if (c > best_c) best_c = c, best_s = s;
   }
-  uint32_t at = best_s;
-  for (uint32_t k = 0; k < G.K; ++k) {
-    G.a[k] = at;
-    G.q[k] = take / G.K + (k < take % G.K ? 1 : 0);
-    G.base[k] = G.entries;
-    G.entries += 1u << (2 * G.q[k]);
-    at += G.q[k];
-  }
+  G.a0 = best_s;
   // Fields of 4 bits (8 classes a word) hold three runs for limits up to 7;
   // otherwise 5 bits (6 classes).  Run 0's entries reach the top bit by
   // themselves; the other runs' caps keep the sum within the field.
@@ -125,17 +136,24 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
       g.hi = std::max(g.hi, at_bulge[i]);
     }
 
+    // Each variant's rank by bulge position within its guide.
+    std::vector<uint32_t> by_place(V);
+    std::vector<uint32_t> at_count;
+    for (const Guide& g : guides) {
+      at_count.assign((size_t)(g.hi - g.lo + 2), 0);
+      for (size_t i = g.begin; i < g.end; ++i) ++at_count[at_bulge[i] - g.lo + 1];
+      for (size_t k = 1; k < at_count.size(); ++k) at_count[k] += at_count[k - 1];
+      for (size_t i = g.begin; i < g.end; ++i) by_place[i] = at_count[at_bulge[i] - g.lo]++;
+    }
+
     // The class of each variant (in generation order) at a level.
     auto classes_of = [&](const Level& lv, std::vector<uint32_t>& cls) {
       cls.assign(V, 0);
       for (size_t gi = 0; gi < guides.size(); ++gi) {
         const Guide& g = guides[gi];
         for (size_t i = g.begin; i < g.end; ++i) {
-          uint32_t part = 0;
-          if (lv.parts > 1) {
-            const int span_g = g.hi - g.lo + 1;
-            part = std::min<uint32_t>(lv.parts - 1, (uint32_t)((at_bulge[i] - g.lo) * (int)lv.parts / span_g));
-          }
+          // The guide's variants in equal shares by bulge position.
+          const uint32_t part = lv.parts > 1 ? by_place[i] * lv.parts / (uint32_t)(g.end - g.begin) : 0u;
           cls[i] = (uint32_t)(gi / lv.guides) * lv.parts + part;
         }
       }
@@ -150,7 +168,8 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
       for (size_t i = 0; i < V; ++i)
         for (uint32_t k = 0; k < G.K; ++k) {
           uint32_t s = 0;
-          for (uint32_t j = 0; j < G.q[k]; ++j) s = s << 4 | bs_class_of((unsigned char)vars[ord[i]]->key[G.a[k] + j]);
+          for (uint32_t j = 0, p = G.a0 + screen_run_at(k); j < screen_run_len(G.K, k) && p + j < L; ++j)
+            s = s << 4 | bs_class_of((unsigned char)vars[ord[i]]->key[p + j]);
           spelled[i * kScreenRuns + k] = s;
         }
     auto pass_rate = [&](const std::vector<size_t>& members) {
@@ -168,10 +187,11 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
         for (uint32_t s : spell)
           for (; s; s >>= 4) concrete += (s & 15) == 0 ? 0.0 : (s & 15) <= 4 ? 1.0 : (s & 15) <= 8 ? 0.3 : 0.6;
         concrete /= (double)spell.size();
-        std::vector<double> next(dist.size() + G.q[k], 0.0);
+        const uint32_t q = screen_run_len(G.K, k);
+        std::vector<double> next(dist.size() + q, 0.0);
         double before = 0;
-        for (uint32_t d = 0; d <= G.q[k]; ++d) {
-          const double cdf = d == G.q[k] ? 1.0 : 1.0 - std::pow(1.0 - binomial_cdf(concrete, (int)d), (double)spell.size());
+        for (uint32_t d = 0; d <= q; ++d) {
+          const double cdf = d == q ? 1.0 : 1.0 - std::pow(1.0 - binomial_cdf(concrete, (int)d), (double)spell.size());
           for (size_t j = 0; j < dist.size(); ++j) next[j + d] += dist[j] * (cdf - before);
           before = cdf;
         }
@@ -181,8 +201,13 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
       for (size_t j = 0; j < dist.size() && j <= lim; ++j) p += dist[j];
       return p;
     };
-    // Issue slots per 32 candidates: the lookups of every word, then for each
-    // candidate that passes a class about 20 and 16 more per 32 variants.
+    // Share of random windows that match the PAM, per strand.
+    double share[2] = {1.0, 1.0};
+    for (uint32_t st = 0; st < 2; ++st)
+      for (uint32_t j = 0; j < (st ? pat.nr : pat.nf); ++j)
+        share[st] *= (4 - __builtin_popcount((st ? pat.rm[j] : pat.fm[j]) & 15u)) / 4.0;
+    const double c = (share[0] + share[1]) * 2048.0;
+    const bool may_scan = can_scan(pat, share[0], share[1]);
     double best = 1e300;
     uint32_t best_level = 0;
     std::vector<std::pair<double, uint32_t>> costs;
@@ -210,20 +235,21 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
         if (m.empty()) continue;
         const double p = pass_rate(m);
         rate += p;
-        work += p * (20.0 + 16.0 * (double)((m.size() + 31) / 32));
+        work += p * (5.0 + 9.0 * (double)((m.size() + 31) / 32));  // clocks to count a passing candidate
         ++sampled;
       }
       if (!sampled) continue;
-      const double words = (double)((n + G.fields - 1) / G.fields);
-      const double cost = words * (28.0 + 9.0 * G.K) + 32.0 * work / sampled * n;
+      const double words = (double)((n + G.fields - 1) / G.fields), queue = queue_cost(c, words);
+      const double cost = (may_scan ? std::min(queue, scan_cost(c, words)) : queue) + c * work / sampled * n;
       costs.emplace_back(cost, li);
       if (cost < best) best = cost, best_level = li;
     }
     if (costs.empty()) return;
-    // The bit-sliced comparer, in the same unit: its table build and, per
-    // variant, half an update step for chained variants or half a full count.
+    // The bit-sliced comparer, in clocks per 32 candidates: its table build
+    // and the count (measured: 100 for 1 variant, 104 for 217 and 1,650 for
+    // 1,000 without bulges).
     const bool chained = V >= 4 * guides.size();
-    const double sliced = 110.0 + (chained ? 0.58 : 1.7) * (double)std::max<size_t>(V, 32);
+    const double sliced = finder_cost(c) + c / 32 * (60.0 + (chained ? 0.5 : 1.6) * (double)std::max<size_t>(V, 32));
     if (force_level < 0 && best >= sliced) return;
     std::stable_sort(costs.begin(), costs.end());
     for (const auto& c : costs)
@@ -233,6 +259,7 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
     // Records by class, class by class.
     const uint32_t n = classes_of(kLevels[best_level], cls);
     G.words = (n + G.fields - 1) / G.fields;
+    plan.scans = may_scan && scan_cost(c, G.words) < queue_cost(c, G.words);
     std::vector<uint32_t> start((size_t)G.words * G.fields + 1, 0);
     for (size_t i = 0; i < V; ++i) ++start[cls[i] + 1];
     for (size_t c = 1; c < start.size(); ++c) start[c] += start[c - 1];

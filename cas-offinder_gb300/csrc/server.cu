@@ -251,12 +251,15 @@ cof_status run_step(cof_server* s, uint64_t k) {
   // at most two oriented candidates per start position of a segment
   COF_CUDA(h, h->queue[0].ensure(2 * s->seg_words * 32 * 4));
   COF_CUDA(h, h->queue[1].ensure(2 * s->seg_words * 32 * 4));
+  cof_status ls = ensure_screen_list(h, std::min<uint64_t>(n, s->seg_words * 32));
+  if (ls) return ls;
   uint64_t count = 0;
   for (;;) {
     COF_CUDA(h, cudaMemsetAsync(h->qcounts.p, 0, 2 * nq * 4, h->stream));
     COF_CUDA(h, cudaMemsetAsync(s->step_count.p, 0, 8, h->stream));
     COF_CUDA(h, cudaEventRecord(h->ev_start, h->stream));
     COF_CUDA(h, cudaStreamWaitEvent(h->stream2, h->ev_start, 0));
+    const HitSink sink{s->step_hits.as<uint64_t>(), s->step_count.as<unsigned long long>(), cap};
     uint64_t pass = 0;
     for (uint64_t si = 0; si < k; ++si)
     for (size_t gi = 0; gi < T.groups.size(); ++gi) {
@@ -268,13 +271,16 @@ cof_status run_step(cof_server* s, uint64_t k) {
       if (w0 >= w1 || g.gids.empty()) continue;
       const int b = (int)(pass & 1);
       uint32_t* qc = h->qcounts.as<uint32_t>() + si * T.groups.size() + gi;
+      if (g.screen_scans) {
+        launch_group_scan(h, g, w0, w1, qc, sink);
+        continue;
+      }
       uint32_t* q = h->queue[b].as<uint32_t>();
       if (pass >= 2) COF_CUDA(h, cudaStreamWaitEvent(h->stream2, h->ev_used[b], 0));
       launch_finder(gv, w0, w1, g.fpat, q, qc, h->stream2);
       COF_CUDA(h, cudaEventRecord(h->ev_found[b], h->stream2));
       COF_CUDA(h, cudaStreamWaitEvent(h->stream, h->ev_found[b], 0));
-      launch_group_compare(gv, g, q, qc, qc + nq, w0 * 32, s->step_hits.as<uint64_t>(),
-                           s->step_count.as<unsigned long long>(), cap, h->sm_count, h->stream);
+      launch_group_compare(h, g, q, qc, qc + nq, w0 * 32, sink);
       COF_CUDA(h, cudaEventRecord(h->ev_used[b], h->stream));
       ++pass;
     }

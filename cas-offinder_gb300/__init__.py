@@ -438,8 +438,8 @@ class CasOFFinder:
         return mm_loci[:k].copy(), mm_count[:k].copy(), direction[:k].tobytes()
 
     def set_comparer(self, kind):
-        """0 auto (table screen where it pays, else bit-sliced when it fits), 1
-        popcount, 2 bit-sliced when it fits."""
+        """0 auto (table screen or direct count where they pay, else bit-sliced
+        when it fits), 1 popcount, 2 bit-sliced when it fits."""
         self._check(self._L.cof_set_comparer(self._h, kind))
 
     def set_autotune(self, on=True):
@@ -455,7 +455,7 @@ class CasOFFinder:
     def comparer_info(self):
         k, sl = ctypes.c_int(), ctypes.c_int()
         self._check(self._L.cof_comparer_info(self._h, ctypes.byref(k), ctypes.byref(sl)))
-        return {"kind": {1: "popcount", 2: "bit-sliced", 3: "screen"}[k.value], "slots": sl.value}
+        return {"kind": {1: "popcount", 2: "bit-sliced", 3: "screen", 4: "direct"}[k.value], "slots": sl.value}
 
     # instrumentation
     def set_profiling(self, on=True):

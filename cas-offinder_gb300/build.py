@@ -35,7 +35,7 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompil
               "--expt-relaxed-constexpr", *ARCH]
 CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-Wall", "-Wno-unused-function"]
 
-CU_SOURCES = ["kernels.cu", "screen.cu", "screen_plan.cu", "comparer_bs.cu", "engine.cu", "server.cu", "noalloc.cu"]
+CU_SOURCES = ["kernels.cu", "screen.cu", "screen_plan.cu", "direct.cu", "comparer_bs.cu", "engine.cu", "server.cu", "noalloc.cu"]
 CPP_SOURCES = ["input.cpp", "genome_io.cpp", "synth.cpp", "router.cpp", "gzip_out.cpp"]
 # comparer_bs_inst.cu is compiled once per (table row words, window words,
 # concrete-only) instance set of the bit-sliced comparer.

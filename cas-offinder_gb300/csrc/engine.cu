@@ -428,8 +428,16 @@ void build_group_host(int kind, PatternGroup& g, const std::vector<const Variant
   const size_t V = vars.size();
   if (kind == 0) plan_screen(vars, g.gids, g.fpat, -1, gh.screen);
   else gh.screen = ScreenPlan();
+  // A few variants may be cheaper to count at every start.
+  g.direct_on = false;
+  if (kind == 0 && V >= 1 && V <= (size_t)kDirectVariants) {
+    std::vector<DirectVariant> dv;
+    for (size_t i = 0; i < V; ++i) dv.push_back(DirectVariant{vars[i]->key, g.gids[i], vars[i]->threshold});
+    g.direct_on = plan_direct(g.pattern, dv.data(), V, g.direct) && direct_cost(g.direct) <= gh.screen.cost;
+    if (g.direct_on) gh.screen = ScreenPlan();
+  }
   adopt_screen(g, gh.screen);
-  if (g.screen_on) {
+  if (g.screen_on || g.direct_on) {
     g.screen_levels = gh.screen.candidates;
     g.nonN_sum = 0;
     for (const Variant* v : vars) g.nonN_sum += (double)(v->key.size() - std::count(v->key.begin(), v->key.end(), 'N'));
@@ -482,6 +490,7 @@ cof_status upload_screen(cof_handle* h, const ScreenPlan& plan, int nw, DevBuf& 
 }
 
 cof_status upload_group(cof_handle* h, PatternGroup& g, const GroupHost& gh, cudaStream_t st) {
+  if (g.direct_on) return COF_OK;
   if (g.screen_on) return upload_screen(h, gh.screen, g.nw, g.screen_records, g.screen_first, g.screen_tables, st);
   COF_CUDA(h, g.vmask.ensure(gh.masks.size()));
   COF_CUDA(h, cudaMemcpyAsync(g.vmask.p, gh.masks.data(), gh.masks.size(), cudaMemcpyHostToDevice, st));
@@ -537,6 +546,10 @@ void launch_group_compare(const cof_handle* h, const PatternGroup& g, const uint
 
 void launch_group_scan(const cof_handle* h, const PatternGroup& g, uint64_t w0, uint64_t w1, uint32_t* qc,
                        const HitSink& sink) {
+  if (g.direct_on) {
+    launch_direct(h->genome.view(), w0, w1, g.direct, qc, sink, h->sm_count, h->stream);
+    return;
+  }
   // Equal pieces of at most kScanWords.
   const uint64_t pieces = (w1 - w0 + kScanWords - 1) / kScanWords;
   for (uint64_t i = 0; i < pieces; ++i)
@@ -592,6 +605,7 @@ using namespace cof::eng;
 cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<const Variant*>& vars) {
   g.bs_tuned.clear();
   g.screen_tuned.clear();
+  if (g.direct_on) return COF_OK;
   if (g.screen_on ? g.screen_levels.size() < 2 : !g.bs_slots || g.bs_candidates.size() < 2) return COF_OK;
   const DevGenome& dg = h->genome;
   const uint64_t npos = dg.n >= g.L ? dg.n - g.L + 1 : 0;
@@ -876,7 +890,7 @@ cof_status run_passes(cof_handle* h, uint64_t hit_cap, std::vector<EventPair>& e
       const uint64_t words = (npos + 31) / 32;
       const uint64_t w0 = s * kSegWords, w1 = std::min(words, w0 + kSegWords);
       if (w0 >= w1 || g.gids.empty()) continue;
-      if (g.screen_scans) {
+      if (g.scans()) {
         // The whole genome at once; during a streamed upload, segment by
         // segment as the planes arrive.
         if (s > 0 && !h->upload_pending) continue;
@@ -974,6 +988,8 @@ std::string pass_graph_key(const cof_handle* h, uint64_t cap) {
       put64((uint64_t)p);
     put64(g.screen_on);
     put64(g.screen_scans);
+    put64(g.direct_on);
+    if (g.direct_on) put(&g.direct, sizeof(g.direct));
     put(&g.screen, sizeof(g.screen));
     put(&g.fpat, sizeof(g.fpat));
   }
@@ -1081,7 +1097,7 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
   if (h->job_gid0.back() == 0) return COF_OK;
   bool queues = false, screens = false;
   for (const PatternGroup& g : h->groups) {
-    queues |= !g.screen_scans;
+    queues |= !g.scans();
     screens |= g.screen_on;
   }
   if (queues)
@@ -1835,7 +1851,9 @@ cof_status cof_schedule_text(cof_handle* h, const char** text, size_t* len) {
     char line[256];
     snprintf(line, sizeof line, "%s variants=%zu slots=%d", g.pattern.c_str(), g.gids.size(), g.bs_slots);
     t += line;
-    if (g.screen_on) {
+    if (g.direct_on) {
+      t += " direct";
+    } else if (g.screen_on) {
       snprintf(line, sizeof line, " screen%s %s words=%u runs=%u", g.screen_scans ? " scanning" : "",
                screen_level_name(g.screen_level), g.screen.words, g.screen.K);
       t += line;
@@ -1872,7 +1890,7 @@ cof_status cof_comparer_info(const cof_handle* h, int* kind, int* slots) {
   if (!h) return COF_ERR_ARG;
   int k = 0, sl = 0;
   for (const PatternGroup& g : h->groups) {
-    k = std::max(k, g.screen_on ? 3 : g.bs_slots ? 2 : 1);
+    k = std::max(k, g.direct_on ? 4 : g.screen_on ? 3 : g.bs_slots ? 2 : 1);
     sl = std::max(sl, g.bs_slots);
   }
   if (kind) *kind = k ? k : 1;

@@ -12,6 +12,7 @@
 
 #include "../../include/cof.h"
 #include "cof_internal.h"
+#include "direct.cuh"
 #include "kernels.cuh"
 #include "screen.cuh"
 
@@ -133,6 +134,9 @@ struct PatternGroup {
   std::vector<std::pair<uint32_t, float>> screen_tuned;  // (partition, µs per segment) measured by the autotuner
   DevBuf screen_records, screen_first, screen_tables;
   bool screen_scans = false;  // the screen scans the planes itself: no finder pass, no candidate queue
+  bool direct_on = false;     // direct count (direct.cuh): no tables, no candidates
+  DirectParams direct;
+  bool scans() const { return screen_scans || direct_on; }
   ScreenTables screen_tb() const {
     return ScreenTables{screen_records.as<uint32_t>(), screen_first.as<uint32_t>(), screen_tables.as<uint32_t>()};
   }
@@ -251,8 +255,8 @@ cof_status build_group_tables(cof_handle* h, PatternGroup& g, const std::vector<
 // comparer.  `tile_ctr`: a zeroed u32 of this launch.  Runs on h->stream.
 void launch_group_compare(const cof_handle* h, const PatternGroup& g, const uint32_t* q, const uint32_t* qc,
                           uint32_t* tile_ctr, uint64_t pos0, const HitSink& sink);
-// Scans plane words [w0, w1) for g (screen_scans) on h->stream; candidates
-// are added to *qc.
+// Scans plane words [w0, w1) for g (scans()) on h->stream; candidates are
+// added to *qc.
 void launch_group_scan(const cof_handle* h, const PatternGroup& g, uint64_t w0, uint64_t w1, uint32_t* qc,
                        const HitSink& sink);
 // The list buffers of the screens of launches over up to `positions` starts.

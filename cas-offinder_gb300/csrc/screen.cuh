@@ -61,6 +61,7 @@ constexpr uint32_t screen_record_words(int nw) { return nw == 1 ? 8 : 12; }
 struct ScreenPlan {
   bool on = false;
   bool scans = false;  // the scanning kernel rather than the finder and the screen of its queue
+  double cost = 1e300;  // SM clocks per 2,048 starts of the screen or, where it is ahead, the bit-sliced comparer
   ScreenGeom geom;
   std::vector<uint32_t> records;  // screen_record_words(nw) per variant
   std::vector<uint32_t> first;    // words * (fields + 1): first record of each class of a word, then the word's end

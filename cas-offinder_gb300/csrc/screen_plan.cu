@@ -250,6 +250,7 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
     // 1,000 without bulges).
     const bool chained = V >= 4 * guides.size();
     const double sliced = finder_cost(c) + c / 32 * (60.0 + (chained ? 0.5 : 1.6) * (double)std::max<size_t>(V, 32));
+    plan.cost = std::min(best, sliced);
     if (force_level < 0 && best >= sliced) return;
     std::stable_sort(costs.begin(), costs.end());
     for (const auto& c : costs)

@@ -271,7 +271,7 @@ cof_status run_step(cof_server* s, uint64_t k) {
       if (w0 >= w1 || g.gids.empty()) continue;
       const int b = (int)(pass & 1);
       uint32_t* qc = h->qcounts.as<uint32_t>() + si * T.groups.size() + gi;
-      if (g.screen_scans) {
+      if (g.scans()) {
         launch_group_scan(h, g, w0, w1, qc, sink);
         continue;
       }

@@ -307,15 +307,13 @@ cof_status cof_comparer_chunk(cof_handle* h, const char* chr, uint64_t chrlen, c
  * are host strings of patternlen bytes (the padded pattern and one compare
  * string; reverse complements are formed internally), `stream` a
  * cudaStream_t (0 = default stream).  Work is queued on `stream`; the results
- * are valid once it completes.  The candidate queue is a fixed 16 MiB device
- * array inside the library (held by every GPU that loads it), so n is limited
- * to 2^21 positions: larger chunks return COF_ERR_TOO_LARGE.  The first call
- * on a device looks up that array's device address; make it before any stream
- * capture.  All calls share the array: calls that overlap on the GPU race, so
- * order them (e.g. one stream).  Nothing is allocated or freed.  `pattern` and
+ * are valid once it completes.  n is limited to 2^21 positions: larger chunks
+ * return COF_ERR_TOO_LARGE.  The library keeps no device memory for the call
+ * (candidates are not stored), so calls on different streams may overlap as
+ * long as their outputs differ.  Nothing is allocated or freed.  `pattern` and
  * `comp` are upper-cased first (as the reference upper-cases its input file);
- * the compare string's masks travel as a kernel argument, so nothing on the
- * host is read after the call returns.  If the calling thread already holds an
+ * both strings travel as a kernel argument, so nothing on the host is read
+ * after the call returns.  If the calling thread already holds an
  * unread CUDA error, the call returns COF_ERR_CUDA without queuing work and
  * leaves that error for the caller. */
 cof_status cof_search_chunk_static(const uint32_t* d_hi, const uint32_t* d_lo, const uint32_t* d_ot, uint64_t n,
@@ -332,21 +330,27 @@ uint64_t cof_plane_words(uint64_t n);
 uint64_t cof_pack_text(const char* seq, uint64_t n, uint32_t* hi, uint32_t* lo, uint32_t* ot, uint64_t* exc_pos,
                        uint8_t* exc_byte);
 
-/* ---- comparer selection.  0 (default): the bit-sliced comparer when every
+/* ---- comparer selection.  0 (default): per pattern group the fastest by
+ * the cost model: the table screen (lookups rule out most candidates, the
+ * rest are counted; mismatch limits up to 15), the direct count of every
+ * start (up to 8 compare variants), or the bit-sliced comparer when every
  * compare variant has at most 32 positions that can mismatch, else the
  * popcount comparer; 1: always the popcount comparer; 2: bit-sliced where
- * possible (same as 0).  Both give identical hits. */
+ * possible, else popcount.  All give identical hits. */
 cof_status cof_set_comparer(cof_handle* h, int kind);
 /* Autotuner of the bit-sliced comparer's lane-program length (variants per
- * lane program): on by default; on the first search of a job set it times the
- * comparer on one genome segment for the cost model's best lengths and keeps
- * the fastest.  Off: the cost model alone chooses. */
+ * lane program) and of the screen's split of the variants into classes: on by
+ * default; on the first search of a job set it times the comparer on one
+ * genome segment for the cost model's best choices and keeps the fastest.
+ * Off: the cost model alone chooses. */
 cof_status cof_set_autotune(cof_handle* h, int enable);
 /* One line per pattern group of the last search: pattern, variants, slots,
- * chosen program length m and chunk count, and the autotuner's timings.
+ * the comparer (chosen program length m and chunk count, or the screen's
+ * classes and table words, or "direct"), and the autotuner's timings.
  * Valid until the next call that returns text. */
 cof_status cof_schedule_text(cof_handle* h, const char** text, size_t* len);
-/* Comparer used by the last search: *kind 1 popcount, 2 bit-sliced; *slots =
+/* Comparer used by the last search (the highest of its groups'): *kind 1
+ * popcount, 2 bit-sliced, 3 table screen, 4 direct count; *slots =
  * the bit-sliced slot count (mismatchable positions per variant, padded). */
 cof_status cof_comparer_info(const cof_handle* h, int* kind, int* slots);
 

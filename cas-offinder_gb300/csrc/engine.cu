@@ -799,6 +799,9 @@ cof_status upload_jobs(cof_handle* h) {
   if (!sf.empty())
     COF_CUDA(h, cudaMemcpyAsync(h->sfmt.p, sf.data(), sf.size() * sizeof(ShapeFmt), cudaMemcpyHostToDevice, h->stream));
   if (!pool.empty()) COF_CUDA(h, cudaMemcpyAsync(h->pool.p, pool.data(), pool.size(), cudaMemcpyHostToDevice, h->stream));
+  COF_CUDA(h, h->job_start.ensure(h->job_gid0.size() * 4));
+  COF_CUDA(h, cudaMemcpyAsync(h->job_start.p, h->job_gid0.data(), h->job_gid0.size() * 4, cudaMemcpyHostToDevice,
+                              h->stream));
   COF_CUDA(h, cudaStreamSynchronize(h->stream));
   h->jobs_on_device = true;
   return COF_OK;
@@ -1112,11 +1115,32 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
   // host memory cannot be graph nodes: both run the passes directly.
   const bool graph = h->use_graphs && !h->profiling && (!h->upload_pending || h->upload_pinned);
   if (h->upload_pending && (st = ensure_upload_events(h, h->upload_pending))) return st;
+  const GenomeView gv = h->genome.view();
+  FormatTables ft{h->vfmt.as<VariantFmt>(), h->sfmt.as<ShapeFmt>(), h->pool.as<char>()};
+  // Searches with few hits are finished on the device before the host knows
+  // their count (profiled ones time the general path).
+  constexpr uint64_t kSmallText = 1ull << 20;
+  const bool small = !h->profiling && J <= kSmallJobs;
+  if (small) {
+    for (DevBuf* b : {&h->hits_sorted, &h->row_offsets, &h->row_bytes}) COF_CUDA(h, b->ensure(kSmallHits * 8));
+    COF_CUDA(h, h->small_out.ensure(sizeof(SmallOut)));
+    COF_CUDA(h, h->host_text.ensure(kSmallText + 1));
+  }
+  const SmallOut* so = (const SmallOut*)h->small_out.p;
   for (;;) {
     st = graph ? run_passes_graph(h, cap, &nseg) : run_passes(h, cap, evs, &nseg);
     if (st) return st;
-    COF_CUDA(h, cudaMemcpyAsync(&nhits, h->hit_count.p, 8, cudaMemcpyDeviceToHost, h->stream));
+    if (small) {
+      launch_small_search(gv, ft, h->hits.as<uint64_t>(), h->hit_count.as<unsigned long long>(), cap,
+                          h->job_start.as<uint32_t>(), (uint32_t)J, h->hits_sorted.as<uint64_t>(),
+                          h->row_offsets.as<uint64_t>(), h->row_bytes.as<uint64_t>(), (SmallOut*)h->small_out.p,
+                          (char*)h->host_text.p, kSmallText, h->stream);
+      COF_CUDA(h, cudaGetLastError());
+    } else {
+      COF_CUDA(h, cudaMemcpyAsync(&nhits, h->hit_count.p, 8, cudaMemcpyDeviceToHost, h->stream));
+    }
     COF_CUDA(h, cudaStreamSynchronize(h->stream));
+    if (small) nhits = so->hits;
     if (nhits <= cap) break;
     for (EventPair& p : evs) {  // discard the overflowing pass's timings
       h->event_pool.push_back(p.a);
@@ -1147,13 +1171,26 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
   }
   h->last_hits = nhits;
   if (nhits == 0) return COF_OK;
+  if (small && nhits <= kSmallHits && so->bytes <= kSmallText) {
+    std::copy(so->job_byte0, so->job_byte0 + J + 1, h->job_byte0.begin());
+    ((char*)h->host_text.p)[so->bytes] = 0;
+    h->last_rows = so->rows;
+    if (sink) {
+      if (so->bytes && sink->fn(sink->ctx, (const char*)h->host_text.p, so->bytes) != 0)
+        return fail(h, COF_ERR_IO, "the row writer failed after 0 bytes");
+      sink->written = so->bytes;
+    } else {
+      *rows = (const char*)h->host_text.p;
+      *rows_len = so->bytes;
+    }
+    return h->summary_on ? summarise(h, nhits) : COF_OK;
+  }
   // Sort hit keys into output order.
   COF_CUDA(h, h->hits_sorted.ensure(nhits * 8));
   COF_CUDA(h, h->row_bytes.ensure(nhits * 8));
   COF_CUDA(h, h->row_offsets.ensure(nhits * 8));
   COF_CUDA(h, h->row_count.ensure(nhits * 4));
   COF_CUDA(h, h->small.ensure(64));
-  COF_CUDA(h, h->job_start.ensure((J + 1) * 4));
   COF_CUDA(h, h->job_bytes.ensure((J + 1) * 8));
   // Key bits the order depends on: strand (bit 7), position, variant id up to
   // the largest id in use.  The mismatch bits below never break a tie: a
@@ -1177,8 +1214,6 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
                                              (int64_t)nhits, 7, end_bit, h->stream));
   if ((st = record_stop(h, evs, h->stream))) return st;
   // Row sizes, offsets, per-job byte ranges, then the rows themselves.
-  const GenomeView gv = h->genome.view();
-  FormatTables ft{h->vfmt.as<VariantFmt>(), h->sfmt.as<ShapeFmt>(), h->pool.as<char>()};
   if ((st = record_start(h, evs, "format", (double)nhits, h->stream))) return st;
   launch_row_lengths(gv, ft, h->hits_sorted.as<uint64_t>(), nhits, h->row_bytes.as<uint64_t>(),
                      h->row_count.as<uint32_t>(), h->stream);
@@ -1188,7 +1223,6 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
   tmp = h->sort_tmp.cap;
   COF_CUDA(h, cub::DeviceReduce::Sum(h->sort_tmp.p, tmp, h->row_count.as<uint32_t>(), h->small.as<uint64_t>(),
                                      (int64_t)nhits, h->stream));
-  COF_CUDA(h, cudaMemcpyAsync(h->job_start.p, h->job_gid0.data(), (J + 1) * 4, cudaMemcpyHostToDevice, h->stream));
   launch_job_bounds(h->hits_sorted.as<uint64_t>(), nhits, h->job_start.as<uint32_t>(), (uint32_t)J,
                     h->row_offsets.as<uint64_t>(), h->row_bytes.as<uint64_t>(), h->job_bytes.as<uint64_t>(),
                     h->stream);

@@ -182,7 +182,7 @@ struct cof_handle {
   DevBuf screen_items, screen_counts;  // candidates that passed a screen (ScreenList), used on `stream`
   DevBuf queue[2], qcounts, hits, hits_sorted, summary_counts, hit_count, sort_tmp, row_bytes, row_offsets, row_count, text, small,
       job_start, job_bytes;
-  HostPinned host_text;
+  HostPinned host_text, small_out;  // small_out: SmallOut of the latest search
   DevBuf stream_dev[2];  // cof_search_stream: row chunks on the device / in pinned memory
   HostPinned stream_host[2];
   cudaEvent_t stream_ev[2] = {nullptr, nullptr};

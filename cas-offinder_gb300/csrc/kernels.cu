@@ -435,24 +435,65 @@ __device__ __forceinline__ HitView decode(uint64_t key) {
 
 }  // namespace
 
+// Bytes of the rows of one hit.
+__device__ __forceinline__ uint64_t hit_row_bytes(const GenomeView& g, const FormatTables& ft, const HitView& h,
+                                                  uint32_t& rows) {
+  const VariantFmt* vf = ft.var + h.gid;
+  const uint32_t rec = record_of(g, h.pos);
+  const uint64_t rel = h.pos - g.rec_start[rec];
+  uint64_t bytes = 0;
+  for (uint32_t s = vf->shape_begin[h.strand]; s < vf->shape_end[h.strand]; ++s) {
+    const ShapeFmt sh = ft.shape[s];
+    bytes += sh.head_len + sh.dna_len + g.rec_name_len[rec] + decimal_len(rel + (uint64_t)sh.offset) + 1 +
+             decimal_len(h.mm) + sh.tail_len + 5;  // tabs around chromosome, location, direction, mismatches
+  }
+  rows = vf->shape_end[h.strand] - vf->shape_begin[h.strand];
+  return bytes;
+}
+
 __global__ void row_len_kernel(GenomeView g, FormatTables ft, const uint64_t* __restrict__ hits, uint64_t n_hits,
                                uint64_t* __restrict__ row_bytes, uint32_t* __restrict__ row_count) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_hits) return;
-  const HitView h = decode(hits[i]);
-  const VariantFmt vf = ft.var[h.gid];
-  const uint32_t rec = record_of(g, h.pos);
-  const uint64_t rel = h.pos - g.rec_start[rec];
-  const uint32_t fixed_sep = 5;  // tabs around chromosome, location, direction, mismatches
-  uint64_t bytes = 0;
-  for (uint32_t s = vf.shape_begin[h.strand]; s < vf.shape_end[h.strand]; ++s) {
-    const ShapeFmt sh = ft.shape[s];
-    bytes += sh.head_len + sh.dna_len + g.rec_name_len[rec] + decimal_len(rel + (uint64_t)sh.offset) + 1 +
-             decimal_len(h.mm) + sh.tail_len + fixed_sep;
-  }
-  row_bytes[i] = bytes;
-  row_count[i] = vf.shape_end[h.strand] - vf.shape_begin[h.strand];
+  row_bytes[i] = hit_row_bytes(g, ft, decode(hits[i]), row_count[i]);
 }
+
+// The oriented window of a hit with mismatches lower-cased
+// (indicate_mismatches, cas-offinder.cpp:299-317: byte += 32).
+struct RowWindow {
+  const GenomeView& g;
+  uint64_t H, Lo, O, pos;
+  const char* comp;
+  uint32_t L, strand;
+  __device__ __forceinline__ RowWindow(const GenomeView& g, const FormatTables& ft, const HitView& h)
+      : g(g), pos(h.pos), strand(h.strand) {
+    L = ft.var[h.gid].L;
+    comp = ft.pool + ft.var[h.gid].comp_off;
+    // The window's plane bits, 64 positions from h.pos (three words per plane
+    // cover any L <= 64 at any bit offset).
+    const uint64_t w0 = h.pos >> 5;
+    const unsigned b0 = (unsigned)(h.pos & 31);
+    auto bits64 = [&](const uint32_t* plane) {
+      const uint64_t lo64 = ((uint64_t)plane[w0 + 1] << 32) | plane[w0];
+      return b0 ? (lo64 >> b0) | ((uint64_t)plane[w0 + 2] << (64 - b0)) : lo64;
+    };
+    H = bits64(g.hi), Lo = bits64(g.lo), O = bits64(g.ot);
+  }
+  // Oriented position k of the window, as printed; computed where the DNA
+  // column asks for it (a per-thread window array would live in local
+  // memory).
+  __device__ __forceinline__ unsigned char operator()(uint32_t k) const {
+    const uint32_t q = strand ? L - 1 - k : k;  // window position of oriented position k
+    const unsigned hb = (unsigned)(H >> q) & 1u, lb = (unsigned)(Lo >> q) & 1u;
+    unsigned char c;
+    // Bytes T, C, A, G (and their complements A, G, T, C) packed low to high.
+    if (!((O >> q) & 1u)) c = (unsigned char)((strand ? 0x43544741u : 0x47414354u) >> (8 * (hb * 2 + lb)));
+    else if (!hb) c = lb ? ';' : 'N';  // complement_byte leaves both as they are
+    else c = strand ? dev_complement(genome_byte(g, pos + q)) : genome_byte(g, pos + q);
+    if (dev_mismatch((unsigned char)comp[k], c)) c = (unsigned char)(c + 32);
+    return c;
+  }
+};
 
 // Rows of one hit at `o` (the bytes row_len_kernel counted).
 __device__ __forceinline__ void write_row(const GenomeView& g, const FormatTables& ft, uint64_t key, char* o) {
@@ -460,34 +501,8 @@ __device__ __forceinline__ void write_row(const GenomeView& g, const FormatTable
   // Fields read in place: a local copy of the struct, indexed by strand,
   // would live in local memory.
   const VariantFmt* vf = ft.var + h.gid;
-  const uint32_t L = vf->L;
-  const char* comp = ft.pool + vf->comp_off;
   const uint32_t s_begin = vf->shape_begin[h.strand], s_end = vf->shape_end[h.strand];
-  // Oriented window with mismatches lower-cased (indicate_mismatches,
-  // cas-offinder.cpp:299-317: byte += 32).
-  // The window's plane bits, 64 positions from h.pos (three words per plane
-  // cover any L <= 64 at any bit offset).
-  const uint64_t w0 = h.pos >> 5;
-  const unsigned b0 = (unsigned)(h.pos & 31);
-  auto bits64 = [&](const uint32_t* plane) {
-    const uint64_t lo64 = ((uint64_t)plane[w0 + 1] << 32) | plane[w0];
-    return b0 ? (lo64 >> b0) | ((uint64_t)plane[w0 + 2] << (64 - b0)) : lo64;
-  };
-  const uint64_t H = bits64(g.hi), Lo = bits64(g.lo), O = bits64(g.ot);
-  // Oriented position k of the window, as printed; computed where the DNA
-  // column asks for it (a per-thread window array would live in local
-  // memory).
-  auto win = [&](uint32_t k) {
-    const uint32_t q = h.strand ? L - 1 - k : k;  // window position of oriented position k
-    const unsigned hb = (unsigned)(H >> q) & 1u, lb = (unsigned)(Lo >> q) & 1u;
-    unsigned char c;
-    // Bytes T, C, A, G (and their complements A, G, T, C) packed low to high.
-    if (!((O >> q) & 1u)) c = (unsigned char)((h.strand ? 0x43544741u : 0x47414354u) >> (8 * (hb * 2 + lb)));
-    else if (!hb) c = lb ? ';' : 'N';  // complement_byte leaves both as they are
-    else c = h.strand ? dev_complement(genome_byte(g, h.pos + q)) : genome_byte(g, h.pos + q);
-    if (dev_mismatch((unsigned char)comp[k], c)) c = (unsigned char)(c + 32);
-    return c;
-  };
+  const RowWindow win(g, ft, h);
   const uint32_t rec = record_of(g, h.pos);
   const uint64_t rel = h.pos - g.rec_start[rec];
   const char* name = g.rec_names + g.rec_name_off[rec];
@@ -566,6 +581,164 @@ void launch_write_rows(const GenomeView& g, const FormatTables& ft, const uint64
   if (!n_hits) return;
   write_rows_kernel<<<(unsigned)((n_hits + kRowThreads - 1) / kRowThreads), kRowThreads, 0, stream>>>(
       g, ft, hits, n_hits, offsets, base, end, out);
+}
+
+namespace {
+
+constexpr int kSmallThreads = 1024;
+
+// One CTA: sorts the keys (bitonic, in shared memory), scans the row bytes.
+// A search with a handful of hits is bound by its launches and round trips:
+// this replaces a sort, three scans and reductions, their set-up kernels and
+// two waits of the host.
+__global__ void __launch_bounds__(kSmallThreads) small_sort_kernel(
+    const __grid_constant__ GenomeView g, const __grid_constant__ FormatTables ft, const uint64_t* __restrict__ hits,
+    const unsigned long long* __restrict__ hit_count, uint64_t hit_cap, const uint32_t* __restrict__ job_gid0,
+    uint32_t njobs, uint64_t* __restrict__ sorted, uint64_t* __restrict__ offsets, uint64_t* __restrict__ row_bytes,
+    SmallOut* __restrict__ out) {
+  __shared__ uint64_t key[kSmallHits];
+  __shared__ uint64_t at[kSmallHits + 1];
+  __shared__ uint64_t warp_sum[32];
+  __shared__ unsigned long long all_rows;
+  const uint64_t n64 = *hit_count;
+  const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  if (n64 > kSmallHits || n64 > hit_cap) {
+    if (t == 0) out->hits = n64, out->bytes = ~0ull;
+    return;
+  }
+  const uint32_t n = (uint32_t)n64;
+  uint32_t m = 2;
+  while (m < n) m *= 2;
+  if (t == 0) all_rows = 0;
+  for (uint32_t i = t; i < m; i += kSmallThreads) key[i] = i < n ? hits[i] : ~0ull;
+  __syncthreads();
+  for (uint32_t k = 2; k <= m; k *= 2)
+    for (uint32_t j = k / 2; j > 0; j /= 2) {
+      for (uint32_t i = t; i < m / 2; i += kSmallThreads) {
+        const uint32_t a = (i & ~(j - 1)) * 2 + (i & (j - 1)), b = a + j;
+        const uint64_t x = key[a], y = key[b];
+        if ((x > y) == ((a & k) == 0)) key[a] = y, key[b] = x;
+      }
+      __syncthreads();
+    }
+  // Two hits per thread, neighbours in order.
+  uint64_t mine[2] = {0, 0};
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (2 * t + i < n) {
+      const uint64_t x = key[2 * t + i];
+      uint32_t rows;
+      mine[i] = hit_row_bytes(g, ft, decode(x), rows);
+      sorted[2 * t + i] = x;
+      atomicAdd(&all_rows, (unsigned long long)rows);
+    }
+  uint64_t incl = mine[0] + mine[1];
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint64_t v = __shfl_up_sync(kFull, incl, d);
+    if (lane >= (uint32_t)d) incl += v;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    uint64_t v = warp_sum[lane];
+    const uint64_t own = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint64_t x = __shfl_up_sync(kFull, v, d);
+      if (lane >= (uint32_t)d) v += x;
+    }
+    warp_sum[lane] = v - own;
+  }
+  __syncthreads();
+  const uint64_t first = warp_sum[warp] + incl - mine[0] - mine[1];
+  at[2 * t] = first;
+  at[2 * t + 1] = first + mine[0];
+  if (t == kSmallThreads - 1) at[kSmallHits] = first + mine[0] + mine[1];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (2 * t + i < n) {
+      offsets[2 * t + i] = at[2 * t + i];
+      row_bytes[2 * t + i] = mine[i];
+    }
+  const uint64_t total = at[kSmallHits];
+  for (uint32_t j = t; j <= njobs; j += kSmallThreads) {
+    uint32_t a = 0, z = n;
+    if (j == njobs) {
+      a = n;
+    } else {
+      const uint64_t from = (uint64_t)job_gid0[j] << 44;
+      while (a < z) {
+        const uint32_t mid = (a + z) >> 1;
+        if (key[mid] < from) a = mid + 1;
+        else z = mid;
+      }
+    }
+    out->job_byte0[j] = a < n ? at[a] : total;
+  }
+  if (t == 0) out->hits = n, out->rows = all_rows, out->bytes = total;
+}
+
+// One warp per hit; a lane writes every 32nd byte of a row, so a row's bytes
+// leave in whole sectors.  (The bulk writer's one thread per hit takes 16 us
+// for any number of rows.)
+constexpr int kSmallRowThreads = 256;
+__global__ void __launch_bounds__(kSmallRowThreads) small_rows_kernel(
+    const __grid_constant__ GenomeView g, const __grid_constant__ FormatTables ft,
+    const unsigned long long* __restrict__ hit_count, uint64_t hit_cap, const uint64_t* __restrict__ sorted,
+    const uint64_t* __restrict__ offsets, const uint64_t* __restrict__ row_bytes, char* __restrict__ text,
+    uint64_t text_cap) {
+  const uint64_t n = *hit_count;
+  const uint32_t i = (blockIdx.x * kSmallRowThreads + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (n > kSmallHits || n > hit_cap || i >= n || offsets[n - 1] + row_bytes[n - 1] > text_cap) return;
+  const HitView h = decode(sorted[i]);
+  const VariantFmt* vf = ft.var + h.gid;
+  const RowWindow win(g, ft, h);
+  const uint32_t rec = record_of(g, h.pos);
+  const uint64_t rel = h.pos - g.rec_start[rec];
+  const char* name = g.rec_names + g.rec_name_off[rec];
+  const uint32_t name_len = g.rec_name_len[rec], mm_len = decimal_len(h.mm);
+  char* o = text + offsets[i];
+  // Digit k of a number of `len` digits.
+  auto digit = [](uint64_t v, uint32_t len, uint32_t k) {
+    for (uint32_t d = len - 1 - k; d; --d) v = v <= 0xFFFFFFFFull ? (uint32_t)v / 10u : v / 10;
+    return (char)('0' + v % 10);
+  };
+  for (uint32_t s = vf->shape_begin[h.strand]; s < vf->shape_end[h.strand]; ++s) {
+    const ShapeFmt sh = ft.shape[s];
+    const uint64_t loc = rel + (uint64_t)sh.offset;
+    const uint32_t loc_len = decimal_len(loc);
+    const uint32_t dna = sh.head_len, chr = dna + sh.dna_len + 1, at_loc = chr + name_len + 1, dir = at_loc + loc_len + 1,
+                   mm = dir + 2, tail = mm + mm_len + 1, end = tail + sh.tail_len;
+    for (uint32_t j = lane; j < end; j += 32) {
+      char c;
+      if (j < dna) c = ft.pool[sh.head_off + j];
+      else if (j < chr - 1) {
+        const unsigned char d = (unsigned char)ft.pool[sh.dna_off + j - dna];
+        c = (char)(d >= 0x80 ? win(d - 0x80u) : d);
+      } else if (j >= chr && j < at_loc - 1) c = name[j - chr];
+      else if (j >= at_loc && j < dir - 1) c = digit(loc, loc_len, j - at_loc);
+      else if (j == dir) c = sh.dir;
+      else if (j >= mm && j < tail - 1) c = digit(h.mm, mm_len, j - mm);
+      else if (j >= tail) c = ft.pool[sh.tail_off + j - tail];
+      else c = '\t';
+      o[j] = c;
+    }
+    o += end;
+  }
+}
+
+}  // namespace
+
+void launch_small_search(const GenomeView& g, const FormatTables& ft, const uint64_t* hits,
+                         const unsigned long long* hit_count, uint64_t hit_cap, const uint32_t* job_gid0, uint32_t njobs,
+                         uint64_t* sorted, uint64_t* offsets, uint64_t* row_bytes, SmallOut* out, char* text,
+                         uint64_t text_cap, cudaStream_t stream) {
+  small_sort_kernel<<<1, kSmallThreads, 0, stream>>>(g, ft, hits, hit_count, hit_cap, job_gid0, njobs, sorted, offsets,
+                                                     row_bytes, out);
+  small_rows_kernel<<<kSmallHits * 32 / kSmallRowThreads, kSmallRowThreads, 0, stream>>>(
+      g, ft, hit_count, hit_cap, sorted, offsets, row_bytes, text, text_cap);
 }
 
 // Byte offset of each job's first row: job j's hits start at the first sorted

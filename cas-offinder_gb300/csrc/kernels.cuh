@@ -166,6 +166,22 @@ uint64_t write_rows_wave_hits(int sm_count);
 void launch_write_rows(const GenomeView& g, const FormatTables& ft, const uint64_t* hits, uint64_t n_hits,
                        const uint64_t* offsets, uint64_t base, uint64_t end, char* out, cudaStream_t stream);
 
+// Searches with few hits: sort, row offsets, per-job byte ranges and the rows
+// themselves, without the host knowing the hit count.  When *hit_count is at
+// most kSmallHits (and hit_cap) and the rows take at most text_cap bytes, the
+// sorted keys are left in `sorted`, the rows in `text` (host memory the device
+// can write); otherwise only out->hits (and out->bytes) are set.  `out` lies
+// in such memory too.  offsets / row_bytes: kSmallHits u64 each.
+constexpr uint32_t kSmallHits = 2048, kSmallJobs = 1023;
+struct SmallOut {
+  uint64_t hits, rows, bytes;
+  uint64_t job_byte0[kSmallJobs + 1];
+};
+void launch_small_search(const GenomeView& g, const FormatTables& ft, const uint64_t* hits,
+                         const unsigned long long* hit_count, uint64_t hit_cap, const uint32_t* job_gid0, uint32_t njobs,
+                         uint64_t* sorted, uint64_t* offsets, uint64_t* row_bytes, SmallOut* out, char* text,
+                         uint64_t text_cap, cudaStream_t stream);
+
 // Per job (global variant ids job_gid0[j] .. job_gid0[j+1]), the byte offset
 // of its first row in the formatted text; out[njobs] = total bytes.
 void launch_job_bounds(const uint64_t* sorted, uint64_t n, const uint32_t* job_gid0, uint32_t njobs,

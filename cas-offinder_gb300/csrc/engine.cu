@@ -476,40 +476,52 @@ void build_group_host(int kind, PatternGroup& g, const std::vector<const Variant
                       &g.bs_candidates);
 }
 
-// Copies a planned screen's records and fills its tables on `st`.
-cof_status upload_screen(cof_handle* h, const ScreenPlan& plan, int nw, DevBuf& records, DevBuf& first, DevBuf& tables,
-                         cudaStream_t st) {
-  COF_CUDA(h, records.ensure(plan.records.size() * 4));
-  COF_CUDA(h, first.ensure(plan.first.size() * 4));
+// Fills a planned screen's tables on `st`, behind the copies of its records.
+cof_status fill_screen(cof_handle* h, const ScreenPlan& plan, int nw, DevBuf& records, DevBuf& first, DevBuf& tables,
+                       cudaStream_t st) {
   COF_CUDA(h, tables.ensure((size_t)plan.geom.words * screen_entries(plan.geom.K) * 4));
-  COF_CUDA(h, cudaMemcpyAsync(records.p, plan.records.data(), plan.records.size() * 4, cudaMemcpyHostToDevice, st));
-  COF_CUDA(h, cudaMemcpyAsync(first.p, plan.first.data(), plan.first.size() * 4, cudaMemcpyHostToDevice, st));
   launch_screen_tables(plan.geom, nw, records.as<uint32_t>(), first.as<uint32_t>(), tables.as<uint32_t>(), st);
   COF_CUDA(h, cudaGetLastError());
   return COF_OK;
 }
 
-cof_status upload_group(cof_handle* h, PatternGroup& g, const GroupHost& gh, cudaStream_t st) {
-  if (g.direct_on) return COF_OK;
-  if (g.screen_on) return upload_screen(h, gh.screen, g.nw, g.screen_records, g.screen_first, g.screen_tables, st);
-  COF_CUDA(h, g.vmask.ensure(gh.masks.size()));
-  COF_CUDA(h, cudaMemcpyAsync(g.vmask.p, gh.masks.data(), gh.masks.size(), cudaMemcpyHostToDevice, st));
-  if (g.bs_slots) {
-    COF_CUDA(h, g.bs_prog.ensure(gh.prog.size() * 4));
-    COF_CUDA(h, g.bs_pgid.ensure(gh.pgid.size() * 4));
-    COF_CUDA(h, cudaMemcpyAsync(g.bs_prog.p, gh.prog.data(), gh.prog.size() * 4, cudaMemcpyHostToDevice, st));
-    COF_CUDA(h, cudaMemcpyAsync(g.bs_pgid.p, gh.pgid.data(), gh.pgid.size() * 4, cudaMemcpyHostToDevice, st));
+// The copies of a group's tables.
+void add_group(Upload& up, PatternGroup& g, const GroupHost& gh) {
+  if (g.direct_on) return;
+  if (g.screen_on) {
+    up.add(g.screen_records, gh.screen.records.data(), gh.screen.records.size() * 4);
+    up.add(g.screen_first, gh.screen.first.data(), gh.screen.first.size() * 4);
+    return;
   }
-  return COF_OK;
+  up.add(g.vmask, gh.masks.data(), gh.masks.size());
+  if (g.bs_slots) {
+    up.add(g.bs_prog, gh.prog.data(), gh.prog.size() * 4);
+    up.add(g.bs_pgid, gh.pgid.data(), gh.pgid.size() * 4);
+  }
 }
 
-cof_status build_group_tables(cof_handle* h, PatternGroup& g, const std::vector<const Variant*>& vars) {
-  GroupHost gh;
-  build_group_host(h->comparer_kind, g, vars, gh);
-  cof_status st = upload_group(h, g, gh, h->stream);
-  if (st) return st;
-  // The host vectors die on return: wait for the copies.
-  COF_CUDA(h, cudaStreamSynchronize(h->stream));
+cof_status upload_group(cof_handle* h, PatternGroup& g, const GroupHost& gh, cudaStream_t st) {
+  Upload up;
+  add_group(up, g, gh);
+  for (const Upload::Part& p : up.parts) {
+    COF_CUDA(h, p.dst->ensure(std::max<size_t>(p.bytes, 1)));
+    COF_CUDA(h, cudaMemcpyAsync(p.dst->p, p.src, p.bytes, cudaMemcpyHostToDevice, st));
+  }
+  return g.screen_on ? fill_screen(h, gh.screen, g.nw, g.screen_records, g.screen_first, g.screen_tables, st) : COF_OK;
+}
+
+cof_status Upload::run(cof_handle* h, HostPinned& stage, cudaStream_t st) {
+  size_t total = 0;
+  for (const Part& p : parts) total += (p.bytes + 255) & ~(size_t)255;
+  COF_CUDA(h, stage.ensure(total));
+  char* at = (char*)stage.p;
+  for (const Part& p : parts) {
+    COF_CUDA(h, p.dst->ensure(std::max<size_t>(p.bytes, 1)));
+    if (!p.bytes) continue;
+    std::memcpy(at, p.src, p.bytes);
+    COF_CUDA(h, cudaMemcpyAsync(p.dst->p, at, p.bytes, cudaMemcpyHostToDevice, st));
+    at += (p.bytes + 255) & ~(size_t)255;
+  }
   return COF_OK;
 }
 
@@ -630,18 +642,24 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
   for (cudaEvent_t& e : ev) COF_CUDA(h, cudaEventCreate(&e));
   float best_us = 1e30f;
   if (g.screen_on) {
-    // The screen's partitions, each timed with tables of its own.
+    // The screen's partitions, each timed with its tables in tune_bufs; the
+    // best one's go to the group's own buffers.
     ScreenPlan best_plan;
-    DevBuf best_buf[3];
+    DevBuf(&buf)[3] = h->tune_bufs;
     cof_status ts = COF_OK;
     for (uint32_t level : g.screen_levels) {
       ScreenPlan plan;
       plan_screen(vars, g.gids, g.fpat, (int)level, plan);
       if (!plan.on) continue;
-      DevBuf buf[3];
       float us = 1e30f;
       auto run = [&]() -> cof_status {
-        cof_status st = upload_screen(h, plan, g.nw, buf[0], buf[1], buf[2], h->stream);
+        COF_CUDA(h, buf[0].ensure(plan.records.size() * 4));
+        COF_CUDA(h, buf[1].ensure(plan.first.size() * 4));
+        COF_CUDA(h, cudaMemcpyAsync(buf[0].p, plan.records.data(), plan.records.size() * 4, cudaMemcpyHostToDevice,
+                                    h->stream));
+        COF_CUDA(h, cudaMemcpyAsync(buf[1].p, plan.first.data(), plan.first.size() * 4, cudaMemcpyHostToDevice,
+                                    h->stream));
+        cof_status st = fill_screen(h, plan, g.nw, buf[0], buf[1], buf[2], h->stream);
         if (st) return st;
         for (int rep = 0; rep < 2; ++rep) {
           COF_CUDA(h, cudaMemsetAsync(h->hit_count.p, 0, 8, h->stream));
@@ -669,16 +687,19 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
       if (us < best_us) {
         best_us = us;
         best_plan = std::move(plan);
-        for (int i = 0; i < 3; ++i) best_buf[i] = std::move(buf[i]);
       }
     }
     for (cudaEvent_t e : ev) cudaEventDestroy(e);
     if (ts) return ts;
     if (best_plan.on && best_plan.level != g.screen_level) {
       adopt_screen(g, best_plan);
-      g.screen_records = std::move(best_buf[0]);
-      g.screen_first = std::move(best_buf[1]);
-      g.screen_tables = std::move(best_buf[2]);
+      COF_CUDA(h, cudaStreamSynchronize(h->stream));  // the last timed pass, and copies out of the stage
+      Upload up;
+      up.add(g.screen_records, best_plan.records.data(), best_plan.records.size() * 4);
+      up.add(g.screen_first, best_plan.first.data(), best_plan.first.size() * 4);
+      cof_status st = up.run(h, h->stage, h->stream);
+      if (!st) st = fill_screen(h, best_plan, g.nw, g.screen_records, g.screen_first, g.screen_tables, h->stream);
+      return st;
     }
     return COF_OK;
   }
@@ -747,7 +768,9 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
 
 cof_status upload_jobs(cof_handle* h) {
   if (h->jobs_on_device) return COF_OK;
-  h->groups.clear();
+  // The new batch's groups take over the old one's device buffers.
+  std::vector<PatternGroup> old;
+  old.swap(h->groups);
   h->job_gid0.assign(1, 0);
   for (const Job& job : h->jobs) {
     if (job.pattern.size() > (size_t)kMaxL)
@@ -780,10 +803,33 @@ cof_status upload_jobs(cof_handle* h) {
   std::vector<ShapeFmt> sf;
   for (const Job& job : h->jobs) append_format_tables(job, vf, sf, pool);
   if (pool.size() >= (1ull << 32)) return fail(h, COF_ERR_UNSUPPORTED, "row tables exceed 4 GB");
+  Upload up;
+  std::vector<GroupHost> gh(h->groups.size());
   for (size_t gi = 0; gi < h->groups.size(); ++gi) {
-    cof_status st = build_group_tables(h, h->groups[gi], group_vars[gi]);
-    if (st) return st;
+    PatternGroup& g = h->groups[gi];
+    if (gi < old.size())
+      for (DevBuf PatternGroup::*b : {&PatternGroup::vmask, &PatternGroup::bs_prog, &PatternGroup::bs_pgid,
+                                      &PatternGroup::screen_records, &PatternGroup::screen_first,
+                                      &PatternGroup::screen_tables})
+        g.*b = std::move(old[gi].*b);
+    build_group_host(h->comparer_kind, g, group_vars[gi], gh[gi]);
+    add_group(up, g, gh[gi]);
   }
+  old.clear();
+  up.add(h->vfmt, vf.data(), vf.size() * sizeof(VariantFmt));
+  up.add(h->sfmt, sf.data(), sf.size() * sizeof(ShapeFmt));
+  up.add(h->pool, pool.data(), pool.size());
+  up.add(h->job_start, h->job_gid0.data(), h->job_gid0.size() * 4);
+  // Earlier searches have waited for their work, copies out of the stage
+  // among it, unless one failed.
+  COF_CUDA(h, cudaStreamSynchronize(h->stream));
+  cof_status st = up.run(h, h->stage, h->stream);
+  for (size_t gi = 0; gi < h->groups.size() && !st; ++gi) {
+    PatternGroup& g = h->groups[gi];
+    if (g.screen_on)
+      st = fill_screen(h, gh[gi].screen, g.nw, g.screen_records, g.screen_first, g.screen_tables, h->stream);
+  }
+  if (st) return st;
   // The planes of a streamed upload are not resident yet: such a search
   // keeps the cost model's choice.
   if (h->autotune && !h->upload_pending)
@@ -791,18 +837,6 @@ cof_status upload_jobs(cof_handle* h) {
       cof_status st = autotune_group(h, h->groups[gi], group_vars[gi]);
       if (st) return st;
     }
-  COF_CUDA(h, h->vfmt.ensure(std::max<size_t>(total, 1) * sizeof(VariantFmt)));
-  COF_CUDA(h, h->sfmt.ensure(std::max<size_t>(sf.size(), 1) * sizeof(ShapeFmt)));
-  COF_CUDA(h, h->pool.ensure(std::max<size_t>(pool.size(), 1)));
-  if (total)
-    COF_CUDA(h, cudaMemcpyAsync(h->vfmt.p, vf.data(), total * sizeof(VariantFmt), cudaMemcpyHostToDevice, h->stream));
-  if (!sf.empty())
-    COF_CUDA(h, cudaMemcpyAsync(h->sfmt.p, sf.data(), sf.size() * sizeof(ShapeFmt), cudaMemcpyHostToDevice, h->stream));
-  if (!pool.empty()) COF_CUDA(h, cudaMemcpyAsync(h->pool.p, pool.data(), pool.size(), cudaMemcpyHostToDevice, h->stream));
-  COF_CUDA(h, h->job_start.ensure(h->job_gid0.size() * 4));
-  COF_CUDA(h, cudaMemcpyAsync(h->job_start.p, h->job_gid0.data(), h->job_gid0.size() * 4, cudaMemcpyHostToDevice,
-                              h->stream));
-  COF_CUDA(h, cudaStreamSynchronize(h->stream));
   h->jobs_on_device = true;
   return COF_OK;
 }

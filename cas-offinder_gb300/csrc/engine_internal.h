@@ -182,6 +182,8 @@ struct cof_handle {
   DevBuf screen_items, screen_counts;  // candidates that passed a screen (ScreenList), used on `stream`
   DevBuf queue[2], qcounts, hits, hits_sorted, summary_counts, hit_count, sort_tmp, row_bytes, row_offsets, row_count, text, small,
       job_start, job_bytes;
+  DevBuf tune_bufs[3];  // a screen's records, classes and tables while its partitions are timed
+  HostPinned stage;  // page-locked source of the batch's tables (Upload)
   HostPinned host_text, small_out;  // small_out: SmallOut of the latest search
   DevBuf stream_dev[2];  // cof_search_stream: row chunks on the device / in pinned memory
   HostPinned stream_host[2];
@@ -228,8 +230,6 @@ bool make_finder_pattern(const std::string& fwd, const std::string& rev, FinderP
 std::string revcomp(const std::string& s);
 // Initialises g (pattern, L, word count, finder pattern) for a padded pattern.
 void init_group(PatternGroup& g, const std::string& pattern);
-// Builds and uploads g's comparer tables for its variants `vars` (g.gids
-// already set, one id per variant).  Synchronizes h->stream.
 // Pool of pinned host buffers kept by the handle: acquire returns a buffer of
 // at least `bytes` (its size in *cap), or nullptr; release gives it back.
 // Thread-safe.
@@ -246,10 +246,22 @@ struct GroupHost {
 // `vars` (ids g.gids); `kind` as cof_set_comparer.  Thread-safe: touches only
 // its arguments.
 void build_group_host(int kind, PatternGroup& g, const std::vector<const Variant*>& vars, GroupHost& gh);
+// Host-to-device copies gathered into one page-locked buffer, so that they are
+// queued without waiting.  The sources may go once `run` returns.
+struct Upload {
+  struct Part {
+    DevBuf* dst;
+    const void* src;
+    size_t bytes;
+  };
+  std::vector<Part> parts;
+  void add(DevBuf& dst, const void* src, size_t bytes) { parts.push_back(Part{&dst, src, bytes}); }
+  // Copies every part on `st` by way of `stage`, whose earlier copies are done.
+  cof_status run(cof_handle* h, HostPinned& stage, cudaStream_t st);
+};
 // Copies `gh` into g's device buffers on `st`; gh must stay alive until the
 // copies are done.
 cof_status upload_group(cof_handle* h, PatternGroup& g, const GroupHost& gh, cudaStream_t st);
-cof_status build_group_tables(cof_handle* h, PatternGroup& g, const std::vector<const Variant*>& vars);
 // Compares the candidates of one finder pass (queue `q`, count `qc`, segment
 // starting at `pos0`) with g's variants: screen, bit-sliced or popcount
 // comparer.  `tile_ctr`: a zeroed u32 of this launch.  Runs on h->stream.

@@ -1,6 +1,7 @@
 // Host side of the table screen (see screen.cuh): where its runs lie, how the
 // variants are split into classes, and whether it pays.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 
@@ -33,6 +34,16 @@ double binomial_cdf(double c, int d) {
     p *= 3.0 * (n - k) / (k + 1);
   }
   return std::min(1.0, s);
+}
+
+// Class row of a pattern byte (bs_class_of), by table.
+uint32_t class_of(char c) {
+  static const std::array<uint8_t, 256> table = [] {
+    std::array<uint8_t, 256> t{};
+    for (int i = 0; i < 256; ++i) t[i] = (uint8_t)bs_class_of((unsigned char)i);
+    return t;
+  }();
+  return table[(unsigned char)c];
 }
 
 // A guide: a run of variants in generation order.
@@ -77,7 +88,7 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
   std::vector<uint32_t> cover(L, 0);
   for (const Variant* v : vars)
     for (uint32_t k = 0; k < L; ++k) {
-      const uint32_t cl = bs_class_of((unsigned char)v->key[k]);
+      const uint32_t cl = class_of(v->key[k]);
       cover[k] += cl != 0;
       if (cl > 4) G.degenerate = 1;
     }
@@ -146,40 +157,35 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
       for (size_t i = g.begin; i < g.end; ++i) by_place[i] = at_count[at_bulge[i] - g.lo]++;
     }
 
+    // The guide's variants in equal shares by bulge position.
+    auto part_of = [&](const Level& lv, const Guide& g, size_t i) {
+      return lv.parts > 1 ? by_place[i] * lv.parts / (uint32_t)(g.end - g.begin) : 0u;
+    };
     // The class of each variant (in generation order) at a level.
     auto classes_of = [&](const Level& lv, std::vector<uint32_t>& cls) {
       cls.assign(V, 0);
       for (size_t gi = 0; gi < guides.size(); ++gi) {
         const Guide& g = guides[gi];
-        for (size_t i = g.begin; i < g.end; ++i) {
-          // The guide's variants in equal shares by bulge position.
-          const uint32_t part = lv.parts > 1 ? by_place[i] * lv.parts / (uint32_t)(g.end - g.begin) : 0u;
-          cls[i] = (uint32_t)(gi / lv.guides) * lv.parts + part;
-        }
+        for (size_t i = g.begin; i < g.end; ++i) cls[i] = (uint32_t)(gi / lv.guides) * lv.parts + part_of(lv, g, i);
       }
       return (uint32_t)((guides.size() + lv.guides - 1) / lv.guides) * lv.parts;
     };
-    // Chance that a random candidate passes the class of variants `members`
-    // (generation-order indexes): distinct spellings on each run, each run's
-    // least count taken as that of independent spellings.
-    // The classes of the positions of each run, 4 bits each, per variant.
-    std::vector<uint32_t> spelled(V * kScreenRuns), spell;
-    if (force_level < 0)  // the only use is to choose a partition
-      for (size_t i = 0; i < V; ++i)
-        for (uint32_t k = 0; k < G.K; ++k) {
-          uint32_t s = 0;
-          for (uint32_t j = 0, p = G.a0 + screen_run_at(k); j < screen_run_len(G.K, k) && p + j < L; ++j)
-            s = s << 4 | bs_class_of((unsigned char)vars[ord[i]]->key[p + j]);
-          spelled[i * kScreenRuns + k] = s;
-        }
-    auto pass_rate = [&](const std::vector<size_t>& members) {
+    // Chance that a random candidate passes a class that holds `times` guides'
+    // worth of the variants `members` (generation-order indexes): distinct
+    // spellings on each run, each run's least count taken as that of
+    // independent spellings.
+    std::vector<uint32_t> spell;
+    auto pass_rate = [&](const std::vector<size_t>& members, double times) {
       std::vector<double> dist(1, 1.0);  // distribution of the bound
       uint32_t lim = 0;
+      for (size_t i : members) lim = std::max<uint32_t>(lim, vars[ord[i]]->threshold);
       for (uint32_t k = 0; k < G.K; ++k) {
+        const uint32_t q = screen_run_len(G.K, k), at = G.a0 + screen_run_at(k);
         spell.clear();
         for (size_t i : members) {
-          lim = std::max<uint32_t>(lim, vars[ord[i]]->threshold);
-          spell.push_back(spelled[i * kScreenRuns + k]);
+          uint32_t s = 0;  // the class of each position, 4 bits
+          for (uint32_t j = 0; j < q && at + j < L; ++j) s = s << 4 | class_of(vars[ord[i]]->key[at + j]);
+          spell.push_back(s);
         }
         std::sort(spell.begin(), spell.end());
         spell.erase(std::unique(spell.begin(), spell.end()), spell.end());
@@ -187,11 +193,11 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
         for (uint32_t s : spell)
           for (; s; s >>= 4) concrete += (s & 15) == 0 ? 0.0 : (s & 15) <= 4 ? 1.0 : (s & 15) <= 8 ? 0.3 : 0.6;
         concrete /= (double)spell.size();
-        const uint32_t q = screen_run_len(G.K, k);
         std::vector<double> next(dist.size() + q, 0.0);
         double before = 0;
         for (uint32_t d = 0; d <= q; ++d) {
-          const double cdf = d == q ? 1.0 : 1.0 - std::pow(1.0 - binomial_cdf(concrete, (int)d), (double)spell.size());
+          const double cdf =
+              d == q ? 1.0 : 1.0 - std::pow(1.0 - binomial_cdf(concrete, (int)d), times * (double)spell.size());
           for (size_t j = 0; j < dist.size(); ++j) next[j + d] += dist[j] * (cdf - before);
           before = cdf;
         }
@@ -217,27 +223,29 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
       if (force_level >= 0 && (uint32_t)force_level != li) continue;
       if (force_level < 0 && lv.guides > 1 && lv.guides >= 2 * guides.size()) continue;
       if (force_level < 0 && lv.parts > 1 && V < 4 * guides.size()) continue;
-      const uint32_t n = classes_of(lv, cls);
+      const uint32_t n = (uint32_t)((guides.size() + lv.guides - 1) / lv.guides) * lv.parts;
       if ((n + G.fields - 1) / G.fields > kScreenMaxWords) continue;
       if (force_level >= 0) {
         best_level = li;
         costs.emplace_back(0.0, li);
         break;
       }
-      // Up to 6 classes, spread over all, stand for the rest.
-      const uint32_t step = std::max<uint32_t>(1, n / 6);
-      double rate = 0, work = 0;
+      // Up to 4 guides, spread over all, stand for the rest.
+      const size_t step = std::max<size_t>(1, guides.size() / 4);
+      double work = 0;
       uint32_t sampled = 0;
-      std::vector<std::vector<size_t>> members(n / step + 1);
-      for (size_t i = 0; i < V; ++i)
-        if (cls[i] % step == 0) members[cls[i] / step].push_back(i);
-      for (const auto& m : members) {
-        if (m.empty()) continue;
-        const double p = pass_rate(m);
-        rate += p;
-        work += p * (5.0 + 9.0 * (double)((m.size() + 31) / 32));  // clocks to count a passing candidate
-        ++sampled;
-      }
+      for (size_t gi = step / 2; gi < guides.size(); gi += step)
+        for (uint32_t part = 0; part < lv.parts; ++part) {
+          const Guide& g = guides[gi];
+          std::vector<size_t> members;
+          for (size_t i = g.begin; i < g.end; ++i)
+            if (part_of(lv, g, i) == part) members.push_back(i);
+          if (members.empty()) continue;
+          const double times = (double)std::min<size_t>(lv.guides, guides.size());
+          // Clocks to count a passing candidate.
+          work += pass_rate(members, times) * (5.0 + 9.0 * std::ceil((double)members.size() * times / 32));
+          ++sampled;
+        }
       if (!sampled) continue;
       const double words = (double)((n + G.fields - 1) / G.fields), queue = queue_cost(c, words);
       const double cost = (may_scan ? std::min(queue, scan_cost(c, words)) : queue) + c * work / sampled * n;
@@ -254,7 +262,8 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
     if (force_level < 0 && best >= sliced) return;
     std::stable_sort(costs.begin(), costs.end());
     for (const auto& c : costs)
-      if (plan.candidates.size() < 3 && c.first <= 2.5 * best) plan.candidates.push_back(c.second);
+      if (plan.candidates.size() < 2 && c.first <= 1.8 * best) plan.candidates.push_back(c.second);
+    if (!chained) plan.candidates.resize(1);  // whole guides only: the model is close, and timing costs as much as it gains
     plan.level = best_level;
 
     // Records by class, class by class.
@@ -273,12 +282,14 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
     for (size_t i = 0; i < V; ++i) {
       const Variant& v = *vars[ord[i]];
       uint32_t* r = &plan.records[(size_t)start[cls[i]]++ * rec];
-      uint32_t* word2[4] = {r + 8, r + 9, r + 10, r + 11};
       for (uint32_t k = 0; k < L; ++k) {
-        const uint32_t m = class_bits_of((unsigned char)v.key[k]), bit = 1u << (k & 31);
-        for (int b = 0; b < 4; ++b)
-          if (m >> b & 1) (k < 32 ? r[b] : *word2[b]) |= bit;
-        if (m & 16) (k < 32 ? r[4] : r[6]) |= bit;
+        const uint32_t m = class_bits_of((unsigned char)v.key[k]);
+        if (k < 32) {
+          for (int b = 0; b < 5; ++b) r[b] |= (m >> b & 1u) << k;
+        } else {
+          for (int b = 0; b < 4; ++b) r[8 + b] |= (m >> b & 1u) << (k - 32);
+          r[6] |= (m >> 4 & 1u) << (k - 32);
+        }
       }
       r[5] = gids[ord[i]] << 4 | v.threshold;
     }

@@ -422,6 +422,9 @@ void adopt_screen(PatternGroup& g, const ScreenPlan& plan) {
   g.screen = plan.geom;
   g.screen_level = plan.level;
   g.screen_scans = plan.on && plan.scans;
+  g.scan_words = kScanWords;
+  while (g.scan_words > kSegWords && (double)(g.scan_words * 32) * plan.listed > kScreenListed * (double)kSegPositions)
+    g.scan_words /= 2;
 }
 
 void build_group_host(int kind, PatternGroup& g, const std::vector<const Variant*>& vars, GroupHost& gh) {
@@ -562,8 +565,8 @@ void launch_group_scan(const cof_handle* h, const PatternGroup& g, uint64_t w0, 
     launch_direct(h->genome.view(), w0, w1, g.direct, qc, sink, h->sm_count, h->stream);
     return;
   }
-  // Equal pieces of at most kScanWords.
-  const uint64_t pieces = (w1 - w0 + kScanWords - 1) / kScanWords;
+  // Equal pieces of at most scan_words.
+  const uint64_t pieces = (w1 - w0 + g.scan_words - 1) / g.scan_words;
   for (uint64_t i = 0; i < pieces; ++i)
     launch_scan_screen(h->genome.view(), w0 + (w1 - w0) * i / pieces, w0 + (w1 - w0) * (i + 1) / pieces, g.fpat,
                        g.screen, g.screen_tb(), screen_list(h), qc, sink, h->sm_count, h->stream);
@@ -1025,6 +1028,7 @@ std::string pass_graph_key(const cof_handle* h, uint64_t cap) {
       put64((uint64_t)p);
     put64(g.screen_on);
     put64(g.screen_scans);
+    put64(g.scan_words);
     put64(g.direct_on);
     if (g.direct_on) put(&g.direct, sizeof(g.direct));
     put(&g.screen, sizeof(g.screen));

@@ -133,6 +133,7 @@ struct PatternGroup {
   std::vector<uint32_t> screen_levels;                  // partitions worth timing (cost model's best first)
   std::vector<std::pair<uint32_t, float>> screen_tuned;  // (partition, µs per segment) measured by the autotuner
   DevBuf screen_records, screen_first, screen_tables;
+  uint64_t scan_words = kScanWords;  // words of a scanning launch: its list holds what passes
   bool screen_scans = false;  // the screen scans the planes itself: no finder pass, no candidate queue
   bool direct_on = false;     // direct count (direct.cuh): no tables, no candidates
   DirectParams direct;

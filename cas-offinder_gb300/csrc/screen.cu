@@ -738,7 +738,7 @@ void run_scan_screen(const GenomeView& g, uint64_t w_begin, uint64_t w_end, cons
 uint32_t screen_lists(int sm_count) { return (uint32_t)sm_count * (kScreenThreads / 32); }
 
 uint64_t screen_list_items(uint64_t positions) {
-  return std::min<uint64_t>(1ull << 25, std::max<uint64_t>(1ull << 18, positions / 16));
+  return std::min<uint64_t>(1ull << 25, std::max<uint64_t>(1ull << 18, positions / 2));
 }
 
 void launch_screen_tables(const ScreenGeom& geom, int nw, const uint32_t* records, const uint32_t* first,

@@ -61,6 +61,7 @@ constexpr uint32_t screen_record_words(int nw) { return nw == 1 ? 8 : 12; }
 struct ScreenPlan {
   bool on = false;
   bool scans = false;  // the scanning kernel rather than the finder and the screen of its queue
+  double listed = 0;    // candidates expected in the list, per start
   double cost = 1e300;  // SM clocks per 2,048 starts of the screen or, where it is ahead, the bit-sliced comparer
   ScreenGeom geom;
   std::vector<uint32_t> records;  // screen_record_words(nw) per variant
@@ -94,6 +95,11 @@ constexpr uint32_t kOddWindow = 1u << 5;
 // `positions` start positions should have room for.  A warp whose list is
 // full counts its further candidates on the spot, so the size only affects
 // the speed.
+// Half an item per start of a segment (2^26 starts), of which 0.25 leaves room
+// for uneven shares.  A listed item costs up to 20 SM clocks, one counted on
+// the spot 95 (64 guides with 2 DNA and 2 RNA bulges, limit 6, on 2^26 starts:
+// 15.9 ms with room for 0.19 items a start, 12.2 ms with 0.5).
+constexpr double kScreenListed = 0.25;
 uint32_t screen_lists(int sm_count);
 uint64_t screen_list_items(uint64_t positions);
 

@@ -25,15 +25,39 @@ constexpr Level kLevels[] = {{64, 1, "64 guides/class"}, {32, 1, "32 guides/clas
                              {1, 1, "1 class/guide"},    {1, 2, "2 classes/guide"},  {1, 3, "3 classes/guide"}};
 constexpr uint32_t kLevelCount = sizeof(kLevels) / sizeof(kLevels[0]);
 
-// P[mismatches of a random window against c concrete positions <= d].
-double binomial_cdf(double c, int d) {
-  const int n = (int)std::lround(c);
-  double p = std::pow(0.25, n), s = 0;
-  for (int k = 0; k <= std::min(d, n); ++k) {
-    s += p;
-    p *= 3.0 * (n - k) / (k + 1);
+// Random windows to estimate pass rates with: base[r][b][w] has bit j set
+// where position j of run r of window w is base b.
+constexpr uint32_t kWindows = 256;
+constexpr size_t kSampled = 32;
+struct Windows {
+  uint8_t base[4][4][kWindows];
+};
+const Windows& windows() {
+  static const Windows win = [] {
+    Windows x;
+    uint64_t s = 0x9E3779B97F4A7C15ull;
+    for (auto& run : x.base)
+      for (uint32_t w = 0; w < kWindows; ++w) {
+        s = s * 6364136223846793005ull + 1442695040888963407ull;
+        const uint32_t hi = (uint32_t)(s >> 40) & 127u, lo = (uint32_t)(s >> 50) & 127u;
+        for (uint32_t b = 0; b < 4; ++b) run[b][w] = (uint8_t)((b & 2 ? hi : ~hi) & (b & 1 ? lo : ~lo) & 127u);
+      }
+    return x;
+  }();
+  return win;
+}
+
+// least[w] = min(least[w], positions j of run r where window w's base b has
+// bit j of m[b] set).
+void least_counts(const Windows& win, uint32_t r, const uint8_t (&m)[4], uint8_t* least) {
+  const auto& base = win.base[r];
+  for (uint32_t w = 0; w < kWindows; ++w) {
+    uint8_t x = (uint8_t)((m[0] & base[0][w]) | (m[1] & base[1][w]) | (m[2] & base[2][w]) | (m[3] & base[3][w]));
+    x = (uint8_t)(x - ((x >> 1) & 0x55));
+    x = (uint8_t)((x & 0x33) + ((x >> 2) & 0x33));
+    x = (uint8_t)((x + (x >> 4)) & 0x0f);
+    least[w] = std::min(least[w], x);
   }
-  return std::min(1.0, s);
 }
 
 // Class row of a pattern byte (bs_class_of), by table.
@@ -50,6 +74,7 @@ uint32_t class_of(char c) {
 struct Guide {
   size_t begin, end;
   int lo, hi;  // bulge positions in use
+  uint32_t limit;
 };
 
 }  // namespace
@@ -139,9 +164,10 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
     for (size_t i = 0; i < V; ++i) {
       const uint32_t v = ord[i];
       if (i == 0 || (rank[v] >> 32) != (rank[ord[i - 1]] >> 32) || vars[v]->id != vars[ord[i - 1]]->id)
-        guides.push_back(Guide{i, i, 1 << 30, -1});
+        guides.push_back(Guide{i, i, 1 << 30, -1, 0});
       Guide& g = guides.back();
       g.end = i + 1;
+      g.limit = std::max<uint32_t>(g.limit, vars[v]->threshold);
       at_bulge[i] = vars[v]->bulges.empty() ? 0 : std::abs(vars[v]->bulges.front().index);
       g.lo = std::min(g.lo, at_bulge[i]);
       g.hi = std::max(g.hi, at_bulge[i]);
@@ -157,6 +183,10 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
       for (size_t i = g.begin; i < g.end; ++i) by_place[i] = at_count[at_bulge[i] - g.lo]++;
     }
 
+    // Guides of like limits share classes: a class passes what its largest
+    // limit passes.
+    std::stable_sort(guides.begin(), guides.end(), [](const Guide& a, const Guide& b) { return a.limit < b.limit; });
+
     // The guide's variants in equal shares by bulge position.
     auto part_of = [&](const Level& lv, const Guide& g, size_t i) {
       return lv.parts > 1 ? by_place[i] * lv.parts / (uint32_t)(g.end - g.begin) : 0u;
@@ -170,42 +200,94 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
       }
       return (uint32_t)((guides.size() + lv.guides - 1) / lv.guides) * lv.parts;
     };
-    // Chance that a random candidate passes a class that holds `times` guides'
-    // worth of the variants `members` (generation-order indexes): distinct
-    // spellings on each run, each run's least count taken as that of
-    // independent spellings.
-    std::vector<uint32_t> spell;
-    auto pass_rate = [&](const std::vector<size_t>& members, double times) {
-      std::vector<double> dist(1, 1.0);  // distribution of the bound
-      uint32_t lim = 0;
-      for (size_t i : members) lim = std::max<uint32_t>(lim, vars[ord[i]]->threshold);
-      for (uint32_t k = 0; k < G.K; ++k) {
-        const uint32_t q = screen_run_len(G.K, k), at = G.a0 + screen_run_at(k);
-        spell.clear();
-        for (size_t i : members) {
-          uint32_t s = 0;  // the class of each position, 4 bits
-          for (uint32_t j = 0; j < q && at + j < L; ++j) s = s << 4 | class_of(vars[ord[i]]->key[at + j]);
-          spell.push_back(s);
+    // Sampled guides stand for the rest: up to kSampled, evenly spaced.
+    // bound[r][p][w] is the least mismatch count on run r of random window w
+    // over the sample's variants whose bulge lies in sixth p of the guide; a
+    // part of any level is a union of sixths.
+    struct Sample {
+      uint32_t limit;
+      size_t variants[6];
+      std::vector<uint8_t> bound;
+    };
+    std::vector<Sample> samples;
+    {
+      const size_t ns = std::min<size_t>(guides.size(), kSampled);
+      const Windows& win = windows();
+      samples.resize(ns);
+      for (size_t k = 0; k < ns; ++k) {
+        const Guide& g = guides[(2 * k + 1) * guides.size() / (2 * ns)];
+        Sample& s = samples[k];
+        s.limit = g.limit;
+        s.bound.assign(G.K * 6 * kWindows, 8);
+        std::fill(s.variants, s.variants + 6, 0);
+        for (size_t i = g.begin; i < g.end; ++i) {
+          const uint32_t part = by_place[i] * 6 / (uint32_t)(g.end - g.begin);
+          ++s.variants[part];
+          for (uint32_t r = 0; r < G.K; ++r) {
+            const uint32_t q = screen_run_len(G.K, r), at = G.a0 + screen_run_at(r);
+            uint8_t m[4] = {};
+            for (uint32_t j = 0; j < q && at + j < L; ++j) {
+              const uint32_t bits = class_bits_of((unsigned char)vars[ord[i]]->key[at + j]);
+              for (int b = 0; b < 4; ++b) m[b] |= (uint8_t)((bits >> b & 1u) << j);
+            }
+            least_counts(win, r, m, s.bound.data() + (r * 6 + part) * kWindows);
+          }
         }
-        std::sort(spell.begin(), spell.end());
-        spell.erase(std::unique(spell.begin(), spell.end()), spell.end());
-        double concrete = 0;
-        for (uint32_t s : spell)
-          for (; s; s >>= 4) concrete += (s & 15) == 0 ? 0.0 : (s & 15) <= 4 ? 1.0 : (s & 15) <= 8 ? 0.3 : 0.6;
-        concrete /= (double)spell.size();
-        std::vector<double> next(dist.size() + q, 0.0);
-        double before = 0;
-        for (uint32_t d = 0; d <= q; ++d) {
-          const double cdf =
-              d == q ? 1.0 : 1.0 - std::pow(1.0 - binomial_cdf(concrete, (int)d), times * (double)spell.size());
-          for (size_t j = 0; j < dist.size(); ++j) next[j + d] += dist[j] * (cdf - before);
-          before = cdf;
-        }
-        dist.swap(next);
       }
-      double p = 0;
-      for (size_t j = 0; j < dist.size() && j <= lim; ++j) p += dist[j];
-      return p;
+    }
+    // What listing and counting the passing candidates costs at level lv with n
+    // classes: SM clocks per candidate, and items listed per candidate.
+    auto count_work = [&](const Level& lv, uint32_t n, double* items) {
+      const size_t ns = samples.size(), whole = (guides.size() + lv.guides - 1) / lv.guides, span = 6 / lv.parts;
+      const size_t groups = std::min(ns, whole), t = ns / groups;
+      const double more = std::max(1.0, (double)std::min<size_t>(lv.guides, guides.size()) / (double)t);
+      double pass = 0, counts = 0;  // sums of P[class passes], and times its counting steps
+      uint32_t classes = 0;
+      std::vector<uint8_t> least(kWindows);
+      for (size_t k = 0; k < groups; ++k)
+        for (uint32_t p = 0; p < lv.parts; ++p) {
+          // t samples (and `more` - 1 times as many like them) in one class.
+          // A random window's runs are independent, so the bound's
+          // distribution is that of the runs' counts convolved.
+          uint32_t limit = 0;
+          size_t members = 0;
+          std::vector<double> dist(1, 1.0);
+          for (uint32_t r = 0; r < G.K; ++r) {
+            std::fill(least.begin(), least.end(), 8);
+            for (size_t j = 0; j < t; ++j) {
+              const Sample& s = samples[k * t + j];
+              for (size_t x = p * span; x < (p + 1) * span; ++x) {
+                const uint8_t* b = s.bound.data() + (r * 6 + x) * kWindows;
+                for (uint32_t w = 0; w < kWindows; ++w) least[w] = std::min(least[w], b[w]);
+                if (r == 0) members += s.variants[x];
+              }
+              limit = std::max(limit, s.limit);
+            }
+            uint32_t hist[9] = {};
+            for (uint32_t w = 0; w < kWindows; ++w) ++hist[std::min<uint32_t>(least[w], G.cap[r])];
+            std::vector<double> next(dist.size() + 8, 0.0);
+            double at_least = 1.0;
+            uint32_t below = 0;
+            for (uint32_t d = 0; d <= 8; ++d) {
+              below += hist[d];
+              const double left = (double)(kWindows - below) / kWindows, beyond = more > 1.0 ? std::pow(left, more) : left;
+              for (size_t j = 0; j < dist.size(); ++j) next[j + d] += dist[j] * (at_least - beyond);
+              at_least = beyond;
+            }
+            dist.swap(next);
+          }
+          if (!members) continue;
+          double passes = 0;
+          for (size_t j = 0; j < dist.size() && j <= limit; ++j) passes += dist[j];
+          pass += passes;
+          counts += passes * std::ceil((double)members * more / 32);
+          ++classes;
+        }
+      if (!classes) return 0.0;
+      const double words = (double)((n + G.fields - 1) / G.fields);
+      const double q = 1.0 - std::pow(std::max(0.0, 1.0 - pass / classes), n / words);  // an item, per candidate and word
+      *items = q * words;
+      return words * (0.5 * (1.0 - std::pow(1.0 - q, 32.0)) + 4.3 * q) + 3.4 * counts / classes * n;
     };
     // Share of random windows that match the PAM, per strand.
     double share[2] = {1.0, 1.0};
@@ -225,39 +307,20 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
       if (force_level < 0 && lv.parts > 1 && V < 4 * guides.size()) continue;
       const uint32_t n = (uint32_t)((guides.size() + lv.guides - 1) / lv.guides) * lv.parts;
       if ((n + G.fields - 1) / G.fields > kScreenMaxWords) continue;
-      if (force_level >= 0) {
-        best_level = li;
-        costs.emplace_back(0.0, li);
-        break;
-      }
-      // Up to 4 guides, spread over all, stand for the rest.
-      const size_t step = std::max<size_t>(1, guides.size() / 4);
-      double work = 0;
-      uint32_t sampled = 0;
-      for (size_t gi = step / 2; gi < guides.size(); gi += step)
-        for (uint32_t part = 0; part < lv.parts; ++part) {
-          const Guide& g = guides[gi];
-          std::vector<size_t> members;
-          for (size_t i = g.begin; i < g.end; ++i)
-            if (part_of(lv, g, i) == part) members.push_back(i);
-          if (members.empty()) continue;
-          const double times = (double)std::min<size_t>(lv.guides, guides.size());
-          // Clocks to count a passing candidate.
-          work += pass_rate(members, times) * (5.0 + 9.0 * std::ceil((double)members.size() * times / 32));
-          ++sampled;
-        }
-      if (!sampled) continue;
       const double words = (double)((n + G.fields - 1) / G.fields), queue = queue_cost(c, words);
-      const double cost = (may_scan ? std::min(queue, scan_cost(c, words)) : queue) + c * work / sampled * n;
+      double items = 0;
+      const double work = c * count_work(lv, n, &items), listed = c / 2048.0 * items;
+      const double cost = (may_scan ? std::min(queue, scan_cost(c, words)) : queue) + work +
+                          95.0 * 2048.0 * std::max(0.0, listed - kScreenListed);
       costs.emplace_back(cost, li);
-      if (cost < best) best = cost, best_level = li;
+      if (cost < best) best = cost, best_level = li, plan.listed = listed;
     }
     if (costs.empty()) return;
     // The bit-sliced comparer, in clocks per 32 candidates: its table build
-    // and the count (measured: 100 for 1 variant, 104 for 217 and 1,650 for
-    // 1,000 without bulges).
+    // and the count (measured: 108 up to 32 variants; with bulges 131 for 224
+    // and 1,231 for 3,554; without 363 for 256 and 1,250 for 1,000).
     const bool chained = V >= 4 * guides.size();
-    const double sliced = finder_cost(c) + c / 32 * (60.0 + (chained ? 0.5 : 1.6) * (double)std::max<size_t>(V, 32));
+    const double sliced = finder_cost(c) + c / 32 * std::max(108.0, 60.0 + (chained ? 0.36 : 1.2) * (double)V);
     plan.cost = std::min(best, sliced);
     if (force_level < 0 && best >= sliced) return;
     std::stable_sort(costs.begin(), costs.end());
@@ -266,9 +329,13 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
     if (!chained) plan.candidates.resize(1);  // whole guides only: the model is close, and timing costs as much as it gains
     plan.level = best_level;
 
-    // Records by class, class by class.
+    // Records by class, class by class.  The classes are dealt out to the words
+    // in turn, each round one word further on (parts of a guide differ), so
+    // that candidates pass all words alike: each CTA's list is an equal share
+    // of the room.
     const uint32_t n = classes_of(kLevels[best_level], cls);
     G.words = (n + G.fields - 1) / G.fields;
+    for (uint32_t& x : cls) x = (x + x / G.words) % G.words * G.fields + x / G.words;
     plan.scans = may_scan && scan_cost(c, G.words) < queue_cost(c, G.words);
     std::vector<uint32_t> start((size_t)G.words * G.fields + 1, 0);
     for (size_t i = 0; i < V; ++i) ++start[cls[i] + 1];

@@ -58,53 +58,65 @@ cof_status issue_upload(cof_handle* h, size_t upto) {
   return COF_OK;
 }
 
-// Words of chunk c + 1 that segment c's windows read (a window of up to 64
-// positions starting in the chunk's last word ends two words later).
+// Words past its last that a range's windows read (a window of up to 64
+// positions starting in the last word ends two words later).
 constexpr uint64_t kUploadHeadWords = 2;
 
-// Events upload_ev[0 .. n), created outside any stream capture.
-cof_status ensure_upload_events(cof_handle* h, size_t n) {
-  while (h->upload_ev.size() < n) {
+// Ends (in words) of the chunks in which page-locked planes of W words are
+// copied.  A copy costs a few microseconds beside its bytes and a scan of a
+// small range leaves the GPU half empty, so chunks grow to four segments; the
+// first are small to let the scans start, and the last, whose scan nothing
+// hides, half a segment (search of 801 Mbp from page-locked planes: 1.77 ms;
+// 2.09 ms by segment with two words of the next one after each, 72 copies in
+// a captured graph; the bytes alone 1.44 ms).
+std::vector<uint64_t> upload_chunks(uint64_t W) {
+  std::vector<uint64_t> ends;
+  for (uint64_t at = 0; at < W;) {
+    const uint64_t most = kSegWords << std::min<size_t>(2, ends.size() / 2);
+    uint64_t n = std::min(most, std::max(kSegWords / 2, (W - at) / 2 & ~(uint64_t)63));
+    if (W - at < kSegWords) n = W - at > kSegWords / 2 + kUploadHeadWords ? kSegWords / 2 : W - at;
+    ends.push_back(at += n);
+  }
+  return ends;
+}
+
+// Page-locked planes: queues the whole upload on stream3 after the work
+// already on h->stream, with upload_ev[c] recorded behind chunk c.  The copies
+// run back to back at the link's rate, ahead of the scans that wait for them.
+cof_status queue_upload_ahead(cof_handle* h) {
+  DevGenome& dg = h->genome;
+  h->upload_ends = upload_chunks(h->upload_words);
+  while (h->upload_ev.size() < h->upload_ends.size()) {
     cudaEvent_t e = nullptr;
     COF_CUDA(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     h->upload_ev.push_back(e);
   }
+  COF_CUDA(h, cudaEventRecord(h->ev_start, h->stream));
+  COF_CUDA(h, cudaStreamWaitEvent(h->stream3, h->ev_start, 0));
+  uint32_t* dst[3] = {dg.hi.as<uint32_t>(), dg.lo.as<uint32_t>(), dg.ot.as<uint32_t>()};
+  uint64_t at = 0;
+  for (size_t c = 0; c < h->upload_ends.size(); ++c) {
+    const uint64_t end = h->upload_ends[c];
+    for (int p = 0; p < 3; ++p)
+      COF_CUDA(h, cudaMemcpyAsync(dst[p] + at, h->upload_src[p] + at, (end - at) * 4, cudaMemcpyHostToDevice, h->stream3));
+    COF_CUDA(h, cudaEventRecord(h->upload_ev[c], h->stream3));
+    at = end;
+  }
+  h->upload_issued = h->upload_pending;
   return COF_OK;
 }
 
-// Page-locked planes: queues the whole upload on stream3 after the work
-// already on h->stream -- chunk 0, then for each c the first words of chunk
-// c + 1 and the rest of it -- with upload_ev[c] recorded once chunk c and the
-// first words of chunk c + 1 are copied.  The copies then run back to back at
-// the link's rate, ahead of the scans that wait for them.
-cof_status queue_upload_ahead(cof_handle* h) {
-  DevGenome& dg = h->genome;
-  const uint64_t W = h->upload_words;
-  const size_t chunks = h->upload_pending;
-  uint32_t* dst[3] = {dg.hi.as<uint32_t>(), dg.lo.as<uint32_t>(), dg.ot.as<uint32_t>()};
-  auto copy = [&](uint64_t w0, uint64_t w1) -> cof_status {
-    if (w0 >= w1) return COF_OK;
-    for (int p = 0; p < 3; ++p)
-      COF_CUDA(h, cudaMemcpyAsync(dst[p] + w0, h->upload_src[p] + w0, (w1 - w0) * 4, cudaMemcpyHostToDevice,
-                                  h->stream3));
-    return COF_OK;
-  };
-  COF_CUDA(h, cudaStreamWaitEvent(h->stream3, h->ev_start, 0));
-  cof_status st = copy(0, std::min<uint64_t>(W, kSegWords));
-  for (size_t c = 0; c < chunks && st == COF_OK; ++c) {
-    const uint64_t n0 = (c + 1) * kSegWords;                 // chunk c + 1
-    const uint64_t h1 = std::min<uint64_t>(W, n0 + kUploadHeadWords);
-    if ((st = copy(n0, h1))) break;
-    COF_CUDA(h, cudaEventRecord(h->upload_ev[c], h->stream3));
-    st = copy(h1, std::min<uint64_t>(W, n0 + kSegWords));
-  }
-  h->upload_issued = chunks;
-  return st;
+// The chunk that brings the last words that windows starting before word w1
+// read.
+size_t upload_chunk_of(const cof_handle* h, uint64_t w1) {
+  const uint64_t need = std::min(h->upload_words, w1 + kUploadHeadWords);
+  return std::lower_bound(h->upload_ends.begin(), h->upload_ends.end(), need) - h->upload_ends.begin();
 }
 
-// With `streamed` the plane copies are left to the search (run_passes queues
-// them: see queue_upload_ahead and issue_upload): the host planes must stay
-// valid until that search is done.
+// With `streamed` the planes are copied under the search: page-locked ones
+// (h->upload_pinned) are queued here (queue_upload_ahead), others by
+// run_passes (issue_upload).  The host planes must stay valid until both that
+// search and stream3 are done.
 cof_status upload_genome(cof_handle* h, DevGenome& dg, const uint32_t* hi, const uint32_t* lo, const uint32_t* ot,
                          uint64_t n, const uint64_t* exc_pos, const uint8_t* exc_byte, uint64_t n_exc,
                          const std::vector<std::string>& names, const std::vector<uint64_t>& starts,
@@ -157,19 +169,16 @@ cof_status upload_genome(cof_handle* h, DevGenome& dg, const uint32_t* hi, const
     pool += names[i];
   }
   const size_t R = std::min(names.size(), starts.size());
-  COF_CUDA(h, dg.rec_start.ensure(std::max<size_t>(R, 1) * 8));
-  COF_CUDA(h, dg.rec_name_off.ensure(std::max<size_t>(R, 1) * 4));
-  COF_CUDA(h, dg.rec_name_len.ensure(std::max<size_t>(R, 1) * 4));
-  COF_CUDA(h, dg.rec_names.ensure(std::max<size_t>(pool.size(), 1)));
-  if (R) {
-    COF_CUDA(h, cudaMemcpyAsync(dg.rec_start.p, starts.data(), R * 8, cudaMemcpyHostToDevice, h->stream));
-    COF_CUDA(h, cudaMemcpyAsync(dg.rec_name_off.p, off.data(), R * 4, cudaMemcpyHostToDevice, h->stream));
-    COF_CUDA(h, cudaMemcpyAsync(dg.rec_name_len.p, len.data(), R * 4, cudaMemcpyHostToDevice, h->stream));
-  }
-  if (!pool.empty())
-    COF_CUDA(h, cudaMemcpyAsync(dg.rec_names.p, pool.data(), pool.size(), cudaMemcpyHostToDevice, h->stream));
-  // Host vectors above are freed on return: wait for the copies.
-  COF_CUDA(h, cudaStreamSynchronize(h->stream));
+  COF_CUDA(h, cudaStreamSynchronize(h->stream));  // earlier copies out of the stage, and from the caller's arrays
+  Upload up;
+  up.add(dg.rec_start, starts.data(), R * 8);
+  up.add(dg.rec_name_off, off.data(), R * 4);
+  up.add(dg.rec_name_len, len.data(), R * 4);
+  up.add(dg.rec_names, pool.data(), pool.size());
+  cof_status us = up.run(h, h->stage, h->stream);
+  if (us) return us;
+  if (!streamed) COF_CUDA(h, cudaStreamSynchronize(h->stream));  // searches on other streams read these tables too
+  if (streamed && h->upload_pinned && (us = queue_upload_ahead(h))) return us;
   dg.n = n;
   dg.n_exc = n_exc;
   dg.n_rec = (uint32_t)R;
@@ -898,9 +907,11 @@ cof_status run_passes(cof_handle* h, uint64_t hit_cap, std::vector<EventPair>& e
   const GenomeView gv = dg.view();
   const size_t G = h->groups.size();
   uint64_t max_words = 0;
+  bool scanning = false;
   for (const PatternGroup& g : h->groups) {
     const uint64_t npos = dg.n >= g.L ? dg.n - g.L + 1 : 0;
     max_words = std::max(max_words, (npos + 31) / 32);
+    scanning |= g.scans();
   }
   const uint64_t nseg = (max_words + kSegWords - 1) / kSegWords;
   *seg_count = nseg;
@@ -911,47 +922,57 @@ cof_status run_passes(cof_handle* h, uint64_t hit_cap, std::vector<EventPair>& e
   COF_CUDA(h, cudaMemsetAsync(h->hit_count.p, 0, 8, h->stream));
   COF_CUDA(h, cudaEventRecord(h->ev_start, h->stream));
   COF_CUDA(h, cudaStreamWaitEvent(h->stream2, h->ev_start, 0));
-  // A streamed upload from page-locked planes is queued whole on stream3;
-  // from pageable planes it follows the scans (issue_upload below).
+  // A streamed upload from page-locked planes is queued whole on stream3 by
+  // now; from pageable planes it follows the scans (issue_upload below).
   const bool ahead = h->upload_pending && h->upload_pinned;
-  if (ahead) {
-    if (h->upload_ev.size() < h->upload_pending)
-      return fail(h, COF_ERR_STATE, "upload events not created before the passes");
-    cof_status st = queue_upload_ahead(h);
-    if (st) return st;
-  }
+  size_t chunk = 0;  // first chunk not yet scanned
   const HitSink sink{h->hits.as<uint64_t>(), h->hit_count.as<unsigned long long>(), hit_cap};
   uint64_t pass = 0;
   for (uint64_t s = 0; s < nseg; ++s) {
-    bool waited = false;  // h->stream has the planes of segment s of a streamed upload
+    // Scanning groups take the whole genome at once; during a streamed upload
+    // what has arrived when segment s is there, chunk by chunk (a profiled
+    // search, whose launches have one event pair per segment and group, in one
+    // launch).
+    uint64_t from = s * kSegWords, upto = from + kSegWords;
+    size_t last = chunk;
+    if (ahead) {
+      last = upload_chunk_of(h, std::min(upto, max_words)) + 1;
+      from = chunk ? h->upload_ends[chunk - 1] - kUploadHeadWords : 0;
+    }
+    bool waited = false;  // h->stream has the planes of segment s of a streamed upload from pageable planes
+    while (scanning && (ahead ? chunk < last : !waited && (s == 0 || h->upload_pending))) {
+      if (ahead) {
+        chunk = h->profiling ? last : chunk + 1;
+        COF_CUDA(h, cudaStreamWaitEvent(h->stream, h->upload_ev[chunk - 1], 0));
+        upto = h->upload_ends[chunk - 1] - (chunk < h->upload_ends.size() ? kUploadHeadWords : 0);
+      } else if (h->upload_pending) {
+        cof_status st = issue_upload(h, (size_t)s + 2);
+        if (st) return st;
+        COF_CUDA(h, cudaEventRecord(h->ev_start, h->stream2));
+        COF_CUDA(h, cudaStreamWaitEvent(h->stream, h->ev_start, 0));
+      } else {
+        upto = max_words;
+      }
+      waited = true;
+      for (size_t gi = 0; gi < G; ++gi) {
+        const PatternGroup& g = h->groups[gi];
+        const uint64_t npos = dg.n >= g.L ? dg.n - g.L + 1 : 0;
+        const uint64_t w1 = std::min((npos + 31) / 32, upto);
+        if (!g.scans() || from >= w1 || g.gids.empty()) continue;
+        uint32_t* qc = h->qcounts.as<uint32_t>() + s * G + gi;
+        cof_status st = record_start(h, evs, "comparer", (double)(s * G + gi), h->stream);
+        if (st) return st;
+        launch_group_scan(h, g, from, w1, qc, sink);
+        if ((st = record_stop(h, evs, h->stream))) return st;
+      }
+      from = upto;
+    }
     for (size_t gi = 0; gi < G; ++gi) {
       const PatternGroup& g = h->groups[gi];
       const uint64_t npos = dg.n >= g.L ? dg.n - g.L + 1 : 0;
       const uint64_t words = (npos + 31) / 32;
       const uint64_t w0 = s * kSegWords, w1 = std::min(words, w0 + kSegWords);
-      if (w0 >= w1 || g.gids.empty()) continue;
-      if (g.scans()) {
-        // The whole genome at once; during a streamed upload, segment by
-        // segment as the planes arrive.
-        if (s > 0 && !h->upload_pending) continue;
-        if (h->upload_pending && !waited) {
-          if (ahead) {
-            COF_CUDA(h, cudaStreamWaitEvent(h->stream, h->upload_ev[std::min<size_t>(s, h->upload_pending - 1)], 0));
-          } else {
-            cof_status st = issue_upload(h, (size_t)s + 2);
-            if (st) return st;
-            COF_CUDA(h, cudaEventRecord(h->ev_start, h->stream2));
-            COF_CUDA(h, cudaStreamWaitEvent(h->stream, h->ev_start, 0));
-          }
-          waited = true;
-        }
-        uint32_t* qc = h->qcounts.as<uint32_t>() + s * G + gi;
-        cof_status st = record_start(h, evs, "comparer", (double)(s * G + gi), h->stream);
-        if (st) return st;
-        launch_group_scan(h, g, w0, h->upload_pending ? w1 : words, qc, sink);
-        if ((st = record_stop(h, evs, h->stream))) return st;
-        continue;
-      }
+      if (g.scans() || w0 >= w1 || g.gids.empty()) continue;
       const int b = (int)(pass & 1);
       uint32_t* qc = h->qcounts.as<uint32_t>() + s * G + gi;
       uint32_t* q = h->queue[b].as<uint32_t>();
@@ -961,8 +982,7 @@ cof_status run_passes(cof_handle* h, uint64_t hit_cap, std::vector<EventPair>& e
       // it spends queued behind that comparer's CTAs.
       if (h->profiling && pass >= 1) COF_CUDA(h, cudaStreamWaitEvent(h->stream2, h->ev_used[1 - b], 0));
       if (ahead) {
-        // Segment s reads chunk s and the first words of chunk s + 1.
-        COF_CUDA(h, cudaStreamWaitEvent(h->stream2, h->upload_ev[std::min<size_t>(s, h->upload_pending - 1)], 0));
+        COF_CUDA(h, cudaStreamWaitEvent(h->stream2, h->upload_ev[upload_chunk_of(h, w1)], 0));
       } else if (h->upload_pending) {
         // Segment s reads plane words up to w1 + 2 (chunks s and s + 1); its
         // finder follows the copies up to chunk s + 1 on the same stream, and
@@ -987,7 +1007,7 @@ cof_status run_passes(cof_handle* h, uint64_t hit_cap, std::vector<EventPair>& e
   // Row formatting reads the planes: the rest of a streamed upload goes
   // before the join.
   if (ahead) {
-    COF_CUDA(h, cudaStreamWaitEvent(h->stream2, h->upload_ev[h->upload_pending - 1], 0));
+    COF_CUDA(h, cudaStreamWaitEvent(h->stream2, h->upload_ev[h->upload_ends.size() - 1], 0));
   } else if (h->upload_pending) {
     cof_status st = issue_upload(h, h->upload_pending);
     if (st) return st;
@@ -1014,10 +1034,6 @@ std::string pass_graph_key(const cof_handle* h, uint64_t cap) {
   put64(h->qcounts.cap);
   for (const void* p : {h->screen_items.p, h->screen_counts.p}) put64((uint64_t)p);
   put64(h->screen_items.cap);
-  // A streamed upload's copies are part of the graph.
-  put64(h->upload_pending);
-  for (const uint32_t* p : h->upload_src) put64(h->upload_pending ? (uint64_t)p : 0);
-  put64(h->upload_pending ? h->upload_words : 0);
   put64(cap);
   put64((uint64_t)h->sm_count);
   for (const PatternGroup& g : h->groups) {
@@ -1053,11 +1069,6 @@ cof_status run_passes_graph(cof_handle* h, uint64_t cap, uint64_t* nseg) {
     if (h->pass_graph) cudaGraphExecDestroy(h->pass_graph);
     h->pass_graph = nullptr;
     std::vector<EventPair> none;
-    h->upload_issued = 0;  // a streamed upload is captured whole
-    if (h->upload_pending) {
-      cof_status se = ensure_upload_events(h, h->upload_pending);
-      if (se) return se;
-    }
     COF_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     const cof_status st = run_passes(h, cap, none, nseg);
     cudaGraph_t graph = nullptr;
@@ -1077,7 +1088,6 @@ cof_status run_passes_graph(cof_handle* h, uint64_t cap, uint64_t* nseg) {
   }
   *nseg = h->pass_nseg;
   COF_CUDA(h, cudaGraphLaunch(h->pass_graph, h->stream));
-  h->upload_issued = h->upload_pending;  // the graph copies every chunk
   return COF_OK;
 }
 
@@ -1149,10 +1159,9 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
   COF_CUDA(h, h->hits.ensure(cap * 8));
   std::vector<EventPair> evs;
   uint64_t nseg = 0, nhits = 0;
-  // Profiled searches time each launch with events, and copies from pageable
-  // host memory cannot be graph nodes: both run the passes directly.
-  const bool graph = h->use_graphs && !h->profiling && (!h->upload_pending || h->upload_pinned);
-  if (h->upload_pending && (st = ensure_upload_events(h, h->upload_pending))) return st;
+  // Profiled searches time each launch with events, and those under a streamed
+  // upload wait for its copies: both run the passes directly.
+  const bool graph = h->use_graphs && !h->profiling && !h->upload_pending;
   const GenomeView gv = h->genome.view();
   FormatTables ft{h->vfmt.as<VariantFmt>(), h->sfmt.as<ShapeFmt>(), h->pool.as<char>()};
   // Searches with few hits are finished on the device before the host knows
@@ -1635,13 +1644,13 @@ cof_status cof_search_planes(cof_handle* h, const uint32_t* hi, const uint32_t* 
     nm.push_back(names[i] ? names[i] : "");
     st.push_back(starts[i]);
   }
-  cof_status r = upload_genome(h, h->genome, hi, lo, ot, n, exc_pos, exc_byte, n_exc, nm, st, true);
   h->upload_pinned = true;
   for (const uint32_t* p : {hi, lo, ot}) {
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess || a.type != cudaMemoryTypeHost) h->upload_pinned = false;
   }
   cudaGetLastError();  // an unregistered pointer is not an error here
+  cof_status r = upload_genome(h, h->genome, hi, lo, ot, n, exc_pos, exc_byte, n_exc, nm, st, true);
   if (r == COF_OK) r = do_search(h, rows, rows_len);
   // The whole genome stays resident (also when the search stopped early) and
   // the host planes are not read after this call returns.

@@ -543,12 +543,19 @@ ScreenList screen_list(const cof_handle* h) {
   l.items = h->screen_items.as<uint4>();
   l.counts = h->screen_counts.as<uint32_t>();
   l.room = h->screen_items.cap / sizeof(uint4);
+  l.windows = h->screen_windows.as<uint2>();
+  l.odd = h->screen_odd.as<uint32_t>();
   return l;
 }
 }  // namespace
 
-cof_status ensure_screen_list(cof_handle* h, uint64_t positions) {
+cof_status ensure_screen_list(cof_handle* h, uint64_t positions, bool windows) {
   COF_CUDA(h, h->screen_items.ensure(screen_list_items(positions) * sizeof(uint4)));
+  if (windows) {
+    const uint64_t most = 2 * std::min<uint64_t>(kSegPositions, std::max<uint64_t>(positions, 1024));
+    COF_CUDA(h, h->screen_windows.ensure(most * sizeof(uint2)));
+    COF_CUDA(h, h->screen_odd.ensure((most + 31) / 32 * 4));
+  }
   COF_CUDA(h, h->screen_counts.ensure(screen_lists(h->sm_count) * 4));
   return COF_OK;
 }
@@ -638,7 +645,7 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
   const uint64_t w0 = (words / kSegWords / 2) * kSegWords, w1 = std::min(words, w0 + kSegWords);
   if (!g.screen_scans || g.screen_levels.size() > 1) COF_CUDA(h, h->queue[0].ensure(2 * kSegPositions * 4));
   if (g.screen_on) {
-    cof_status st = ensure_screen_list(h, std::min<uint64_t>(dg.n, 32 * kScanWords));
+    cof_status st = ensure_screen_list(h, std::min<uint64_t>(dg.n, 32 * kScanWords), true);
     if (st) return st;
   }
   COF_CUDA(h, h->qcounts.ensure(std::max<size_t>(h->qcounts.cap, 8)));  // count, tile counter
@@ -1032,7 +1039,7 @@ std::string pass_graph_key(const cof_handle* h, uint64_t cap) {
     put64((uint64_t)p);
   put64(h->genome.n);
   put64(h->qcounts.cap);
-  for (const void* p : {h->screen_items.p, h->screen_counts.p}) put64((uint64_t)p);
+  for (const void* p : {h->screen_items.p, h->screen_counts.p, h->screen_windows.p, h->screen_odd.p}) put64((uint64_t)p);
   put64(h->screen_items.cap);
   put64(cap);
   put64((uint64_t)h->sm_count);
@@ -1146,14 +1153,15 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
   h->job_byte0.assign(J + 1, 0);
   if (h->summaries.size() != J) h->summaries.assign(J, {});
   if (h->job_gid0.back() == 0) return COF_OK;
-  bool queues = false, screens = false;
+  bool queues = false, screens = false, windows = false;
   for (const PatternGroup& g : h->groups) {
     queues |= !g.scans();
     screens |= g.screen_on;
+    windows |= g.windows();
   }
   if (queues)
     for (DevBuf& q : h->queue) COF_CUDA(h, q.ensure(2 * kSegPositions * 4));
-  if (screens && (st = ensure_screen_list(h, std::min<uint64_t>(h->genome.n, 32 * kScanWords)))) return st;
+  if (screens && (st = ensure_screen_list(h, std::min<uint64_t>(h->genome.n, 32 * kScanWords), windows))) return st;
   COF_CUDA(h, h->hit_count.ensure(8));
   uint64_t cap = std::max<uint64_t>(h->hits.cap / 8, 1u << 20);
   COF_CUDA(h, h->hits.ensure(cap * 8));

@@ -138,6 +138,8 @@ struct PatternGroup {
   bool direct_on = false;     // direct count (direct.cuh): no tables, no candidates
   DirectParams direct;
   bool scans() const { return screen_scans || direct_on; }
+  // The screen extracts the queue's windows first.
+  bool windows() const { return screen_on && !screen_scans && screen.words >= kWindowWords; }
   ScreenTables screen_tb() const {
     return ScreenTables{screen_records.as<uint32_t>(), screen_first.as<uint32_t>(), screen_tables.as<uint32_t>()};
   }
@@ -180,6 +182,7 @@ struct cof_handle {
   DevBuf vfmt, sfmt, pool;           // row formatting tables over all variants
   DevGenome genome, scratch;
 
+  DevBuf screen_windows, screen_odd;  // windows of a queue's candidates (ScreenList), used on `stream`
   DevBuf screen_items, screen_counts;  // candidates that passed a screen (ScreenList), used on `stream`
   DevBuf queue[2], qcounts, hits, hits_sorted, summary_counts, hit_count, sort_tmp, row_bytes, row_offsets, row_count, text, small,
       job_start, job_bytes;
@@ -272,8 +275,9 @@ void launch_group_compare(const cof_handle* h, const PatternGroup& g, const uint
 // added to *qc.
 void launch_group_scan(const cof_handle* h, const PatternGroup& g, uint64_t w0, uint64_t w1, uint32_t* qc,
                        const HitSink& sink);
-// The list buffers of the screens of launches over up to `positions` starts.
-cof_status ensure_screen_list(cof_handle* h, uint64_t positions);
+// The list buffers of the screens of launches over up to `positions` starts
+// (with `windows`, those of a queue's windows too).
+cof_status ensure_screen_list(cof_handle* h, uint64_t positions, bool windows);
 // Lane programs of the bit-sliced comparer for `vars` (ids `gids`), `S` slots,
 // class rows of `row` words; layout in kernels.cuh.
 // force_m (1-24) replaces the cost model's choice of m; `ranked` (may be

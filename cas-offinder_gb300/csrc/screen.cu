@@ -217,6 +217,42 @@ __device__ __forceinline__ void load_tables(const ScreenGeom& G, const ScreenTab
   __syncthreads();
 }
 
+// Whether an item's window holds a non-base byte.
+template <int NW>
+__device__ __forceinline__ bool odd_window(const GenomeView& g, uint32_t seg_w0, uint32_t x, uint32_t L) {
+  uint32_t o[NW], some = 0;
+  load_plane<NW>(o, g.ot, seg_w0 + (x >> 6), (x >> 1) & 31);
+#pragma unroll
+  for (int i = 0; i < NW; ++i)
+    some |= o[i] & (L >= 32u * (i + 1) ? kFull : L > 32u * i ? (1u << (L & 31)) - 1u : 0u);
+  return some != 0;
+}
+
+// The oriented windows of a queue, for a screen that looks them up once per
+// word.
+template <int NW>
+__global__ void __launch_bounds__(256) windows_kernel(const __grid_constant__ GenomeView g,
+                                                      const uint32_t* __restrict__ queue,
+                                                      const uint32_t* __restrict__ qcount, uint64_t seg_pos0, uint32_t a0,
+                                                      uint32_t L, const __grid_constant__ ScreenList list) {
+  const uint32_t n = *qcount, seg_w0 = (uint32_t)(seg_pos0 >> 5);
+  for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < ((n + 31) & ~31u); i += gridDim.x * 256) {
+    const bool have = i < n;
+    const uint32_t e = have ? __ldg(queue + i) : 0u, w = seg_w0 + (e >> 6), r = (e >> 1) & 31;
+    uint32_t h[NW], l[NW];
+    load_plane<NW>(h, g.hi, w, r);
+    load_plane<NW>(l, g.lo, w, r);
+    orient_plane<NW>(h, e & 1, true, L);
+    orient_plane<NW>(l, e & 1, false, L);
+    const uint32_t odd = __ballot_sync(kFull, have && odd_window<NW>(g, seg_w0, e, L));
+    if ((i & 31) == 0) list.odd[i / 32] = odd;
+    if (have)
+      list.windows[i] = NW == 1 ? make_uint2(h[0], l[0])
+                        : a0 >= 32 ? make_uint2(h[NW - 1] >> (a0 & 31), l[NW - 1] >> (a0 & 31))
+                                   : make_uint2(__funnelshift_r(h[0], h[NW - 1], a0), __funnelshift_r(l[0], l[NW - 1], a0));
+  }
+}
+
 // The screen of a finder pass's queue.  One CTA per SM holds one word's
 // tables in shared memory.  The work -- (word, chunk of candidates),
 // word-major -- is cut into one contiguous share per CTA, so a CTA loads the
@@ -225,7 +261,12 @@ __device__ __forceinline__ void load_tables(const ScreenGeom& G, const ScreenTab
 // of 2^26 starts, 64 + 18 us since) and counted by screen_count_kernel.
 // Bound by issue and by the lookups: 32 lanes at random banks take about 3.5
 // shared-memory wavefronts.  0.88 SM clocks per candidate and word.
-template <int NW, int K, bool DEG>
+// READY takes the windows from windows_kernel, an iteration ahead: the plain
+// form waits for the entries and then for the planes in every word, three
+// quarters of its warps' cycles.  Four sets of 256 guides on 0.8 Gbp (16 to 22
+// words): 8.20 -> 7.19 ms; with 3 or 4 words the extraction costs as much as
+// it saves (272 us for 2^26 starts, 16.8 M candidates, either way).
+template <int NW, int K, bool DEG, bool READY>
 __global__ void __launch_bounds__(kScreenThreads, 1) screen_kernel(
     const __grid_constant__ GenomeView g, const uint32_t* __restrict__ queue, const uint32_t* __restrict__ qcount,
     uint64_t seg_pos0, const __grid_constant__ ScreenGeom G, const __grid_constant__ ScreenTables tb, uint32_t L,
@@ -243,53 +284,76 @@ __global__ void __launch_bounds__(kScreenThreads, 1) screen_kernel(
   const uint32_t word0 = u < u_end ? (uint32_t)(u / spans) : 0u;
   const uint32_t tab_addr = (uint32_t)__cvta_generic_to_shared(tab);
   WarpList out(list);
-  // Whether a candidate's window holds a non-base byte.
-  auto odd = [&](uint32_t x) {
-    uint32_t o[NW], some = 0;
-    load_plane<NW>(o, g.ot, seg_w0 + (x == 0xFFFFFFFFu ? 0u : x >> 6), (x >> 1) & 31);
-#pragma unroll
-    for (int i = 0; i < NW; ++i)
-      some |= o[i] & (L >= 32u * (i + 1) ? kFull : L > 32u * i ? (1u << (L & 31)) - 1u : 0u);
-    return some != 0;
-  };
   while (u < u_end) {
     const uint32_t word = (uint32_t)(u / spans);
     const uint64_t word_u = (uint64_t)word * spans, stop = min(u_end, word_u + spans);
     load_tables(G, tb, word, tab, cls);
+    // The coming iteration's entries and windows.
+    uint32_t next[kPerLane];
+    uint2 next_win[kPerLane];
+    auto fetch = [&](uint64_t s) {
+#pragma unroll
+      for (int j = 0; j < kPerLane; ++j) {
+        const uint32_t i = (uint32_t)(s - word_u) * kWarpSpan + lane + 32 * j;
+        const bool have = s < stop && i < n;
+        next[j] = have ? __ldg(queue + i) : 0xFFFFFFFFu;
+        next_win[j] = have ? __ldg(list.windows + i) : make_uint2(0, 0);
+      }
+    };
+    if (READY) fetch(u + (threadIdx.x >> 5));
     for (uint64_t s = u + (threadIdx.x >> 5); s < stop; s += kScreenThreads / 32) {
       const uint32_t i0 = (uint32_t)(s - word_u) * kWarpSpan + lane;
       uint32_t e[kPerLane], test[kPerLane], h0[kPerLane], l0[kPerLane], any = 0;
+      bool odd[kPerLane];
+      if constexpr (READY) {
 #pragma unroll
-      for (int j = 0; j < kPerLane; ++j) {
-        const uint32_t i = i0 + 32 * j;
-        e[j] = i < n ? __ldg(queue + i) : 0xFFFFFFFFu;
-      }
+        for (int j = 0; j < kPerLane; ++j) {
+          e[j] = next[j];
+          h0[j] = next_win[j].x;
+          l0[j] = next_win[j].y;
+          odd[j] = e[j] != 0xFFFFFFFFu && __ldg(list.odd + (i0 + 32 * j) / 32) >> lane & 1u;
+        }
+        fetch(s + kScreenThreads / 32);
 #pragma unroll
-      for (int j = 0; j < kPerLane; ++j) {
-        const bool have = e[j] != 0xFFFFFFFFu;
-        const uint32_t w = seg_w0 + (have ? e[j] >> 6 : 0u), r = (e[j] >> 1) & 31;
-        uint32_t h[NW], l[NW];
-        load_plane<NW>(h, g.hi, w, r);
-        load_plane<NW>(l, g.lo, w, r);
-        orient_plane<NW>(h, e[j] & 1, true, L);
-        orient_plane<NW>(l, e[j] & 1, false, L);
-        // The window from the screen's first position on (26 positions at most).
-        const uint32_t hr = NW == 1 || G.a0 >= 32 ? h[NW - 1] >> (G.a0 & 31) : __funnelshift_r(h[0], h[NW - 1], G.a0);
-        const uint32_t lr = NW == 1 || G.a0 >= 32 ? l[NW - 1] >> (G.a0 & 31) : __funnelshift_r(l[0], l[NW - 1], G.a0);
-        const uint32_t sum = run_sum<K>(tab_addr, hr, lr);
-        test[j] = ~sum & G.top;
-        if (DEG && odd(e[j])) test[j] = G.top;
-        if (!have) test[j] = 0;
-        any |= test[j];
-        h0[j] = h[0];
-        l0[j] = l[0];
+        for (int j = 0; j < kPerLane; ++j) {
+          const uint32_t a0 = NW == 1 ? G.a0 : 0;
+          test[j] = ~run_sum<K>(tab_addr, h0[j] >> a0, l0[j] >> a0) & G.top;
+          if (DEG && odd[j]) test[j] = G.top;
+          if (e[j] == 0xFFFFFFFFu) test[j] = 0;
+          any |= test[j];
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < kPerLane; ++j) {
+          const uint32_t i = i0 + 32 * j;
+          e[j] = i < n ? __ldg(queue + i) : 0xFFFFFFFFu;
+        }
+#pragma unroll
+        for (int j = 0; j < kPerLane; ++j) {
+          const bool have = e[j] != 0xFFFFFFFFu;
+          const uint32_t w = seg_w0 + (have ? e[j] >> 6 : 0u), r = (e[j] >> 1) & 31;
+          uint32_t h[NW], l[NW];
+          load_plane<NW>(h, g.hi, w, r);
+          load_plane<NW>(l, g.lo, w, r);
+          orient_plane<NW>(h, e[j] & 1, true, L);
+          orient_plane<NW>(l, e[j] & 1, false, L);
+          // The window from the screen's first position on (26 positions at most).
+          const uint32_t hr = NW == 1 || G.a0 >= 32 ? h[NW - 1] >> (G.a0 & 31) : __funnelshift_r(h[0], h[NW - 1], G.a0);
+          const uint32_t lr = NW == 1 || G.a0 >= 32 ? l[NW - 1] >> (G.a0 & 31) : __funnelshift_r(l[0], l[NW - 1], G.a0);
+          test[j] = ~run_sum<K>(tab_addr, hr, lr) & G.top;
+          if (DEG && have && odd_window<NW>(g, seg_w0, e[j], L)) test[j] = G.top;
+          if (!have) test[j] = 0;
+          any |= test[j];
+          h0[j] = h[0];
+          l0[j] = l[0];
+        }
       }
       if (!__any_sync(kFull, any)) continue;
 #pragma unroll
       for (int j = 0; j < kPerLane; ++j) {
         const uint32_t m = __ballot_sync(kFull, test[j] != 0);
         if (!m) continue;
-        const uint32_t flag = test[j] && odd(e[j]) ? kOddWindow : 0u;
+        const uint32_t flag = test[j] && (READY ? odd[j] : odd_window<NW>(g, seg_w0, e[j], L)) ? kOddWindow : 0u;
         if (!out.append(m, e[j], test[j] | flag | (word - word0), h0[j], l0[j]))
           count_now<NW>(g, seg_pos0, e[j], test[j], G.bits, cls, tb.records, L, sink);
       }
@@ -534,7 +598,6 @@ constexpr uint32_t kCountShare = 64;   // warps per screening CTA
 // `n` of them, `pos` their positions.
 template <int NW, int V>
 __device__ __forceinline__ void count_gathered(const uint2* got, const uint32_t* pos, uint32_t n,
-                                               
                                                const uint32_t* __restrict__ records, uint32_t v0, uint32_t v1,
                                                uint64_t pos0, const HitSink& sink) {
   const unsigned lane = threadIdx.x & 31;
@@ -700,9 +763,11 @@ void run_screen(const GenomeView& g, const uint32_t* queue, const uint32_t* qcou
                 const ScreenGeom& geom, const ScreenTables& tb, uint32_t L, const ScreenList& list, const HitSink& sink,
                 int sm_count, cudaStream_t stream) {
   const size_t smem = (size_t)screen_entries(K) * 4;
-  cudaFuncSetAttribute(screen_kernel<NW, K, DEG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  screen_kernel<NW, K, DEG>
-      <<<sm_count, kScreenThreads, smem, stream>>>(g, queue, qcount, seg_pos0, geom, tb, L, list, sink);
+  const bool ready = geom.words >= kWindowWords;
+  auto kernel = ready ? screen_kernel<NW, K, DEG, true> : screen_kernel<NW, K, DEG, false>;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (ready) windows_kernel<NW><<<8 * sm_count, 256, 0, stream>>>(g, queue, qcount, seg_pos0, geom.a0, L, list);
+  kernel<<<sm_count, kScreenThreads, smem, stream>>>(g, queue, qcount, seg_pos0, geom, tb, L, list, sink);
   launch_count(g, seg_pos0, geom, NW, tb, L, list, sm_count, kScreenThreads / 32, 0, qcount, 32 * kPerLane, sink,
                stream);
 }

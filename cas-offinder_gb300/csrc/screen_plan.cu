@@ -85,10 +85,13 @@ namespace {
 
 // Costs in SM clocks per 2,048 starts, of which `c` are candidates (measured
 // at 0.08 and 0.2 candidates per start: 280 and 533 for one scanning word,
-// 227 and 265 for the finder, 0.88 per candidate and word of the queue).
+// 227 and 265 for the finder, 0.88 per candidate and word of the queue, 0.65
+// where its windows are extracted first).
 double scan_cost(double c, double words) { return words * (100.0 + 1.08 * c); }
 double finder_cost(double c) { return 182.0 + 0.22 * c; }
-double queue_cost(double c, double words) { return finder_cost(c) + words * (15.0 + 0.88 * c); }
+double queue_cost(double c, double words) {
+  return finder_cost(c) + (words < kWindowWords ? words * (15.0 + 0.88 * c) : 0.3 * c + words * (15.0 + 0.65 * c));
+}
 
 // The scanning kernel stages up to 320 of 2,048 starts' candidates at a time
 // and takes one-word windows.

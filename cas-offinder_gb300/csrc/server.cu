@@ -251,7 +251,8 @@ cof_status run_step(cof_server* s, uint64_t k) {
   // at most two oriented candidates per start position of a segment
   COF_CUDA(h, h->queue[0].ensure(2 * s->seg_words * 32 * 4));
   COF_CUDA(h, h->queue[1].ensure(2 * s->seg_words * 32 * 4));
-  cof_status ls = ensure_screen_list(h, std::min<uint64_t>(n, s->seg_words * 32));
+  const bool windows = std::any_of(T.groups.begin(), T.groups.end(), [](const PatternGroup& g) { return g.windows(); });
+  cof_status ls = ensure_screen_list(h, std::min<uint64_t>(n, s->seg_words * 32), windows);
   if (ls) return ls;
   uint64_t count = 0;
   for (;;) {

@@ -544,7 +544,6 @@ ScreenList screen_list(const cof_handle* h) {
   l.counts = h->screen_counts.as<uint32_t>();
   l.room = h->screen_items.cap / sizeof(uint4);
   l.windows = h->screen_windows.as<uint2>();
-  l.odd = h->screen_odd.as<uint32_t>();
   return l;
 }
 }  // namespace
@@ -554,13 +553,12 @@ cof_status ensure_screen_list(cof_handle* h, uint64_t positions, bool windows) {
   if (windows) {
     const uint64_t most = 2 * std::min<uint64_t>(kSegPositions, std::max<uint64_t>(positions, 1024));
     COF_CUDA(h, h->screen_windows.ensure(most * sizeof(uint2)));
-    COF_CUDA(h, h->screen_odd.ensure((most + 31) / 32 * 4));
   }
   COF_CUDA(h, h->screen_counts.ensure(screen_lists(h->sm_count) * 4));
   return COF_OK;
 }
 
-void launch_group_compare(const cof_handle* h, const PatternGroup& g, const uint32_t* q, const uint32_t* qc,
+void launch_group_compare(const cof_handle* h, const PatternGroup& g, uint32_t* q, const uint32_t* qc,
                           uint32_t* tile_ctr, uint64_t pos0, const HitSink& sink) {
   const GenomeView gv = h->genome.view();
   if (g.screen_on) {
@@ -1039,7 +1037,7 @@ std::string pass_graph_key(const cof_handle* h, uint64_t cap) {
     put64((uint64_t)p);
   put64(h->genome.n);
   put64(h->qcounts.cap);
-  for (const void* p : {h->screen_items.p, h->screen_counts.p, h->screen_windows.p, h->screen_odd.p}) put64((uint64_t)p);
+  for (const void* p : {h->screen_items.p, h->screen_counts.p, h->screen_windows.p}) put64((uint64_t)p);
   put64(h->screen_items.cap);
   put64(cap);
   put64((uint64_t)h->sm_count);

@@ -182,7 +182,7 @@ struct cof_handle {
   DevBuf vfmt, sfmt, pool;           // row formatting tables over all variants
   DevGenome genome, scratch;
 
-  DevBuf screen_windows, screen_odd;  // windows of a queue's candidates (ScreenList), used on `stream`
+  DevBuf screen_windows;  // windows of a queue's candidates (ScreenList), used on `stream`
   DevBuf screen_items, screen_counts;  // candidates that passed a screen (ScreenList), used on `stream`
   DevBuf queue[2], qcounts, hits, hits_sorted, summary_counts, hit_count, sort_tmp, row_bytes, row_offsets, row_count, text, small,
       job_start, job_bytes;
@@ -269,7 +269,7 @@ cof_status upload_group(cof_handle* h, PatternGroup& g, const GroupHost& gh, cud
 // Compares the candidates of one finder pass (queue `q`, count `qc`, segment
 // starting at `pos0`) with g's variants: screen, bit-sliced or popcount
 // comparer.  `tile_ctr`: a zeroed u32 of this launch.  Runs on h->stream.
-void launch_group_compare(const cof_handle* h, const PatternGroup& g, const uint32_t* q, const uint32_t* qc,
+void launch_group_compare(const cof_handle* h, const PatternGroup& g, uint32_t* q, const uint32_t* qc,
                           uint32_t* tile_ctr, uint64_t pos0, const HitSink& sink);
 // Scans plane words [w0, w1) for g (scans()) on h->stream; candidates are
 // added to *qc.

@@ -229,27 +229,24 @@ __device__ __forceinline__ bool odd_window(const GenomeView& g, uint32_t seg_w0,
 }
 
 // The oriented windows of a queue, for a screen that looks them up once per
-// word.
+// word; entries whose window holds a non-base byte get kOddEntry.
+constexpr uint32_t kOddEntry = 1u << 31;
 template <int NW>
-__global__ void __launch_bounds__(256) windows_kernel(const __grid_constant__ GenomeView g,
-                                                      const uint32_t* __restrict__ queue,
+__global__ void __launch_bounds__(256) windows_kernel(const __grid_constant__ GenomeView g, uint32_t* __restrict__ queue,
                                                       const uint32_t* __restrict__ qcount, uint64_t seg_pos0, uint32_t a0,
                                                       uint32_t L, const __grid_constant__ ScreenList list) {
   const uint32_t n = *qcount, seg_w0 = (uint32_t)(seg_pos0 >> 5);
-  for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < ((n + 31) & ~31u); i += gridDim.x * 256) {
-    const bool have = i < n;
-    const uint32_t e = have ? __ldg(queue + i) : 0u, w = seg_w0 + (e >> 6), r = (e >> 1) & 31;
+  for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+    const uint32_t e = queue[i], w = seg_w0 + (e >> 6), r = (e >> 1) & 31;
     uint32_t h[NW], l[NW];
     load_plane<NW>(h, g.hi, w, r);
     load_plane<NW>(l, g.lo, w, r);
     orient_plane<NW>(h, e & 1, true, L);
     orient_plane<NW>(l, e & 1, false, L);
-    const uint32_t odd = __ballot_sync(kFull, have && odd_window<NW>(g, seg_w0, e, L));
-    if ((i & 31) == 0) list.odd[i / 32] = odd;
-    if (have)
-      list.windows[i] = NW == 1 ? make_uint2(h[0], l[0])
-                        : a0 >= 32 ? make_uint2(h[NW - 1] >> (a0 & 31), l[NW - 1] >> (a0 & 31))
-                                   : make_uint2(__funnelshift_r(h[0], h[NW - 1], a0), __funnelshift_r(l[0], l[NW - 1], a0));
+    if (odd_window<NW>(g, seg_w0, e, L)) queue[i] = e | kOddEntry;
+    list.windows[i] = NW == 1 ? make_uint2(h[0], l[0])
+                      : a0 >= 32 ? make_uint2(h[NW - 1] >> (a0 & 31), l[NW - 1] >> (a0 & 31))
+                                 : make_uint2(__funnelshift_r(h[0], h[NW - 1], a0), __funnelshift_r(l[0], l[NW - 1], a0));
   }
 }
 
@@ -264,8 +261,9 @@ __global__ void __launch_bounds__(256) windows_kernel(const __grid_constant__ Ge
 // READY takes the windows from windows_kernel, an iteration ahead: the plain
 // form waits for the entries and then for the planes in every word, three
 // quarters of its warps' cycles.  Four sets of 256 guides on 0.8 Gbp (16 to 22
-// words): 8.20 -> 7.19 ms; with 3 or 4 words the extraction costs as much as
-// it saves (272 us for 2^26 starts, 16.8 M candidates, either way).
+// words): 8.20 -> 6.82 ms; issue-bound since (71 % of slots).  With 3 or 4 words
+// the extraction costs as much as it saves (272 us for 2^26 starts, 16.8 M
+// candidates, either way).
 template <int NW, int K, bool DEG, bool READY>
 __global__ void __launch_bounds__(kScreenThreads, 1) screen_kernel(
     const __grid_constant__ GenomeView g, const uint32_t* __restrict__ queue, const uint32_t* __restrict__ qcount,
@@ -288,38 +286,35 @@ __global__ void __launch_bounds__(kScreenThreads, 1) screen_kernel(
     const uint32_t word = (uint32_t)(u / spans);
     const uint64_t word_u = (uint64_t)word * spans, stop = min(u_end, word_u + spans);
     load_tables(G, tb, word, tab, cls);
-    // The coming iteration's entries and windows.
+    // The coming iteration's entries and windows (past the last: any).
     uint32_t next[kPerLane];
     uint2 next_win[kPerLane];
     auto fetch = [&](uint64_t s) {
 #pragma unroll
       for (int j = 0; j < kPerLane; ++j) {
-        const uint32_t i = (uint32_t)(s - word_u) * kWarpSpan + lane + 32 * j;
-        const bool have = s < stop && i < n;
-        next[j] = have ? __ldg(queue + i) : 0xFFFFFFFFu;
-        next_win[j] = have ? __ldg(list.windows + i) : make_uint2(0, 0);
+        const uint32_t i = min((uint32_t)(s - word_u) * kWarpSpan + lane + 32 * j, n - 1);
+        next[j] = __ldg(queue + i);
+        next_win[j] = __ldg(list.windows + i);
       }
     };
     if (READY) fetch(u + (threadIdx.x >> 5));
     for (uint64_t s = u + (threadIdx.x >> 5); s < stop; s += kScreenThreads / 32) {
       const uint32_t i0 = (uint32_t)(s - word_u) * kWarpSpan + lane;
       uint32_t e[kPerLane], test[kPerLane], h0[kPerLane], l0[kPerLane], any = 0;
-      bool odd[kPerLane];
       if constexpr (READY) {
 #pragma unroll
         for (int j = 0; j < kPerLane; ++j) {
           e[j] = next[j];
           h0[j] = next_win[j].x;
           l0[j] = next_win[j].y;
-          odd[j] = e[j] != 0xFFFFFFFFu && __ldg(list.odd + (i0 + 32 * j) / 32) >> lane & 1u;
         }
         fetch(s + kScreenThreads / 32);
 #pragma unroll
         for (int j = 0; j < kPerLane; ++j) {
           const uint32_t a0 = NW == 1 ? G.a0 : 0;
           test[j] = ~run_sum<K>(tab_addr, h0[j] >> a0, l0[j] >> a0) & G.top;
-          if (DEG && odd[j]) test[j] = G.top;
-          if (e[j] == 0xFFFFFFFFu) test[j] = 0;
+          if (DEG && e[j] >= kOddEntry) test[j] = G.top;
+          if (i0 + 32 * j >= n) test[j] = 0;
           any |= test[j];
         }
       } else {
@@ -353,9 +348,11 @@ __global__ void __launch_bounds__(kScreenThreads, 1) screen_kernel(
       for (int j = 0; j < kPerLane; ++j) {
         const uint32_t m = __ballot_sync(kFull, test[j] != 0);
         if (!m) continue;
-        const uint32_t flag = test[j] && (READY ? odd[j] : odd_window<NW>(g, seg_w0, e[j], L)) ? kOddWindow : 0u;
-        if (!out.append(m, e[j], test[j] | flag | (word - word0), h0[j], l0[j]))
-          count_now<NW>(g, seg_pos0, e[j], test[j], G.bits, cls, tb.records, L, sink);
+        const uint32_t flag =
+            test[j] && (READY ? e[j] >= kOddEntry : odd_window<NW>(g, seg_w0, e[j], L)) ? kOddWindow : 0u;
+        const uint32_t x = READY ? e[j] & ~kOddEntry : e[j];
+        if (!out.append(m, x, test[j] | flag | (word - word0), h0[j], l0[j]))
+          count_now<NW>(g, seg_pos0, x, test[j], G.bits, cls, tb.records, L, sink);
       }
     }
     u = stop;
@@ -759,7 +756,7 @@ void launch_count(const GenomeView& g, uint64_t pos0, const ScreenGeom& geom, in
 }
 
 template <int NW, int K, bool DEG>
-void run_screen(const GenomeView& g, const uint32_t* queue, const uint32_t* qcount, uint64_t seg_pos0,
+void run_screen(const GenomeView& g, uint32_t* queue, const uint32_t* qcount, uint64_t seg_pos0,
                 const ScreenGeom& geom, const ScreenTables& tb, uint32_t L, const ScreenList& list, const HitSink& sink,
                 int sm_count, cudaStream_t stream) {
   const size_t smem = (size_t)screen_entries(K) * 4;
@@ -813,7 +810,7 @@ void launch_screen_tables(const ScreenGeom& geom, int nw, const uint32_t* record
   else screen_tables_kernel<2><<<grid, 256, 0, stream>>>(geom, records, first, tables);
 }
 
-void launch_screen(const GenomeView& g, const uint32_t* queue, const uint32_t* qcount, uint64_t seg_pos0,
+void launch_screen(const GenomeView& g, uint32_t* queue, const uint32_t* qcount, uint64_t seg_pos0,
                    const ScreenGeom& geom, int nw, const ScreenTables& tb, uint32_t L, const ScreenList& list,
                    const HitSink& sink, int sm_count, cudaStream_t stream) {
   auto run = nw == 1 ? (geom.K == 3 ? (geom.degenerate ? run_screen<1, 3, true> : run_screen<1, 3, false>)

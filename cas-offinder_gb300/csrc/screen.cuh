@@ -89,10 +89,8 @@ struct ScreenList {
   uint64_t room = 0;
   // Windows of a queue's candidates, for screens of kWindowWords words or more:
   // the oriented window's first word of the hi and lo planes (two-word windows:
-  // 32 positions from the screen's first on), and a bit for each that holds a
-  // non-base byte.  Room for a full queue.
+  // 32 positions from the screen's first on).  Room for a full queue.
   uint2* windows = nullptr;
-  uint32_t* odd = nullptr;
 };
 // Words from which on a queue's windows are extracted once, ahead of the
 // lookups (measured: a gain at 16, none at 4).
@@ -128,8 +126,9 @@ struct HitSink {
 void launch_screen_tables(const ScreenGeom& geom, int nw, const uint32_t* records, const uint32_t* first,
                           uint32_t* tables, cudaStream_t stream);
 // Tests every entry of `queue` (count read on the device) against the
-// screen's variants; appends hit keys as launch_comparer does.
-void launch_screen(const GenomeView& g, const uint32_t* queue, const uint32_t* qcount, uint64_t seg_pos0,
+// screen's variants; appends hit keys as launch_comparer does.  May mark
+// entries of the queue.
+void launch_screen(const GenomeView& g, uint32_t* queue, const uint32_t* qcount, uint64_t seg_pos0,
                    const ScreenGeom& geom, int nw, const ScreenTables& tb, uint32_t L, const ScreenList& list,
                    const HitSink& sink, int sm_count, cudaStream_t stream);
 // PAM scan and screen in one kernel, without a candidate queue, for windows

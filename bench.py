@@ -741,15 +741,32 @@ def main():
                  f"comparisons per test; measured LOP3 {rates['lop3'] / 1e12:.2f}, POPC {rates['popc'] / 1e12:.2f} "
                  f"T lane-ops/s")
     traffic = committed_traffic("comparer")
-    issued = issued_roofline(eng, cmp, rates)
+    comparer_roof = {"bound": "int-pipe", "kernel": "comparer", "achieved": achieved, "peak": peak,
+                     "unit": "G base-comparisons/s", "frac": achieved / peak if peak else None, "traffic": traffic,
+                     "peak_basis": basis, "base_comparisons_per_test": mean_nonN,
+                     "issued": issued_roofline(eng, cmp, rates),
+                     "note": "the peak assumes every variant counted in full; the lane programs' update "
+                             "steps cost less per base comparison, so frac can pass 1 -- `issued` is the "
+                             "fraction of the LOP3 pipe the count phase itself occupies"}
+    if cinfo["kind"] in ("screen", "direct"):
+        comparer_roof = dict(screen_roofline(cmp, n, nh), kernel="comparer", traffic=traffic)
     # Finder bytes: 0.375 B of planes read per position scanned plus the 4 B
     # queue entry written per candidate; the profiled search runs each
     # finder launch alone, so its events time the kernel itself.
     fnd = stats["finder"]
     cands = eng.kernel_stats("finder.candidates")["units"]
-    finder_bytes = fnd["units"] * 0.375 + cands * 4
-    finder_gbs = finder_bytes / (fnd["ms"] * 1e-3) / 1e9 if fnd["ms"] else 0.0
-    peaks = load_peaks()
+    # A screen that scans the planes itself has no finder launches.
+    finder_roof = None
+    if fnd["launches"]:
+        peaks = load_peaks()
+        finder_bytes = fnd["units"] * 0.375 + cands * 4
+        finder_gbs = finder_bytes / (fnd["ms"] * 1e-3) / 1e9
+        finder_roof = {"bound": "hbm", "achieved": finder_gbs, "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
+                       "frac": finder_gbs / peaks["hbm_gbs"] if peaks.get("hbm_gbs") else None,
+                       "bytes_per_launch": finder_bytes / fnd["launches"],
+                       "us_per_launch": fnd["ms"] * 1e3 / fnd["launches"],
+                       "basis": "0.375 B per genome position (3 bit planes read) + 4 B per candidate "
+                                "(queue entry written); launches timed alone"}
 
     cpu = None
     workdir = tempfile.mkdtemp(prefix="cof_bench_")
@@ -759,9 +776,10 @@ def main():
         except Exception as e:  # the baseline is reported, never required
             cpu = {"failed": f"{e}"[:300]}
 
-    # Kernels of ours per search (finder and comparer per segment; row
-    # lengths and job bounds once; row writing in one launch per chunk, as
-    # the profiled search counted them), times the timed searches.
+    # Kernels of ours per search, times the timed searches: finder and comparer
+    # launches as the profiled search timed them (a scanning screen's several
+    # launches count as one: a lower bound); row lengths and job bounds once;
+    # row writing in one launch per chunk.
     row_chunks = int(eng.kernel_stats("rows.chunks")["units"])
     launches = args.steps * int(stats["finder"]["launches"] + stats["comparer"]["launches"] +
                                 (2 + row_chunks) * stats["format"]["launches"])
@@ -808,19 +826,8 @@ def main():
                     "planes_h2d_alone_gbs": 3 * W * 4 / (h2d_alone_ms * 1e-3) / 1e9,
                     "d2h_1gb_gbs": {"copy_engine": d2h["dma"] / 1e9, "sm_stores": d2h["sm"] / 1e9,
                                     "two_copy_engines": d2h["dma2"] / 1e9}},
-            "roofline": {"bound": "int-pipe", "kernel": "comparer", "achieved": achieved, "peak": peak,
-                         "unit": "G base-comparisons/s", "frac": achieved / peak if peak else None,
-                         "traffic": traffic,
-                         "peak_basis": basis, "base_comparisons_per_test": mean_nonN, "issued": issued,
-                         "note": "the peak assumes every variant counted in full; the lane programs' update "
-                                 "steps cost less per base comparison, so frac can pass 1 -- `issued` is the "
-                                 "fraction of the LOP3 pipe the count phase itself occupies"},
-            "roofline_finder": {"bound": "hbm", "achieved": finder_gbs, "peak": peaks.get("hbm_gbs"),
-                                "unit": "GB/s", "frac": finder_gbs / peaks["hbm_gbs"] if peaks.get("hbm_gbs")
-                                else None, "bytes_per_launch": finder_bytes / max(fnd["launches"], 1),
-                                "us_per_launch": fnd["ms"] * 1e3 / max(fnd["launches"], 1),
-                                "basis": "0.375 B per genome position (3 bit planes read) + 4 B per candidate "
-                                         "(queue entry written); launches timed alone"},
+            "roofline": comparer_roof,
+            "roofline_finder": finder_roof,
             "kernel_ms_per_step": dict({k: v["ms"] for k, v in stats.items()}, **stages),
             "batched": batched,
             "pam_variety": pam_variety,
@@ -905,8 +912,6 @@ def run_batched(P, eng, lens, rates, args, capture=None):
             "setup_ms": statistics.fmean(setup), "search_ms": statistics.fmean(search),
             "speedup_vs_plain_search_only": statistics.fmean(search) * len(texts) / ms}
     eng.set_autotune(True)
-    achieved = cmp["units"] / (cmp["ms"] * 1e-3) / 1e9 if cmp["ms"] else 0.0
-    peak = rates["lop3"] * 16 / 1e9
     return {
         "workload": "1,024 single-guide input files: spacer 20-24 (2% IUPAC), PAM NGG/NRG, mm 3-6, DNA bulge 0-2, "
                     "RNA bulge 0-1, on the same 3.1 Gbp genome",
@@ -917,9 +922,7 @@ def run_batched(P, eng, lens, rates, args, capture=None):
         "plain_split": split,
         "speedup_vs_plain": (plain_ms * len(texts)) / ms, "kernel_ms_profiled": kernel_ms,
         "comparer_schedule": schedule,
-        "comparer_roofline": {"achieved": achieved, "peak": peak, "unit": "G base-comparisons/s",
-                              "frac": achieved / peak if peak else None,
-                              "issued": issued_roofline(eng, cmp, rates)},
+        "comparer_roofline": comparer_roofline(eng, cmp, rates, schedule, sum(lens), hits),
     }
 
 
@@ -959,8 +962,6 @@ def run_pam_variety(P, eng, lens, rates, args, capture=None):
         eng.search_view()
         seq_ms += eng.timer_stop()
     guides = 256 * len(texts)
-    achieved = cmp["units"] / (cmp["ms"] * 1e-3) / 1e9 if cmp["ms"] else 0.0
-    peak = rates["lop3"] * 16 / 1e9
     return {
         "workload": "4 input files x 256 guides: NNGRRT/21-nt, NNNNGMTT/24-nt, NNAGAAW/20-nt, 5'-TTTV/23-nt spacers, "
                     "mm 4, DNA bulge 1, RNA bulge 1, on the same 3.1 Gbp genome",
@@ -968,9 +969,7 @@ def run_pam_variety(P, eng, lens, rates, args, capture=None):
         "variants": info["variants"], "hits": hits, "rows": rows,
         "sequential_value": guides * gbp / (seq_ms / 1e3), "sequential_ms": seq_ms,
         "speedup_vs_sequential": seq_ms / ms, "kernel_ms_profiled": kernel_ms, "comparer_schedule": schedule,
-        "comparer_roofline": {"achieved": achieved, "peak": peak, "unit": "G base-comparisons/s",
-                              "frac": achieved / peak if peak else None,
-                              "issued": issued_roofline(eng, cmp, rates)},
+        "comparer_roofline": comparer_roofline(eng, cmp, rates, schedule, sum(lens), hits),
     }
 
 
@@ -1012,6 +1011,32 @@ def profile_search(args):
     out.update(workload=args.profile_search, genome_bp=n, schedule=eng.schedule().strip())
     print(json.dumps(out), flush=True)
     eng.close()
+
+
+def screen_roofline(cmp, n, hits):
+    """The table screen (or the direct count) against the bytes it cannot do
+    without: the planes read once and a key written per hit."""
+    peaks = load_peaks()
+    nbytes = 0.375 * n + 8.0 * hits
+    gbs = nbytes / (cmp["ms"] * 1e-3) / 1e9 if cmp["ms"] else 0.0
+    return {"bound": "hbm", "achieved": gbs, "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
+            "frac": gbs / peaks["hbm_gbs"] if peaks.get("hbm_gbs") else None,
+            "bytes": nbytes, "equivalent_base_comparisons_g_per_s": cmp["units"] / (cmp["ms"] * 1e-3) / 1e9
+            if cmp["ms"] else None,
+            "note": "bytes: planes read once + 8 B per hit; the kernels are bound by instruction issue "
+                    "(PAM test, table lookups and their listing per candidate), not by these bytes. "
+                    "equivalent_base_comparisons: what counting every variant of every candidate in full would take"}
+
+
+def comparer_roofline(eng, cmp, rates, schedule, n, hits):
+    """Roofline of a batch's comparer launches: the LOP3 pipe where all groups
+    count every variant, the bytes where some are screened."""
+    if " screen " in schedule or " direct" in schedule:
+        return screen_roofline(cmp, n, hits)
+    achieved = cmp["units"] / (cmp["ms"] * 1e-3) / 1e9 if cmp["ms"] else 0.0
+    peak = rates["lop3"] * 16 / 1e9
+    return {"achieved": achieved, "peak": peak, "unit": "G base-comparisons/s",
+            "frac": achieved / peak if peak else None, "issued": issued_roofline(eng, cmp, rates)}
 
 
 def issued_roofline(eng, cmp, rates):

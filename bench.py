@@ -749,7 +749,9 @@ def main():
                              "steps cost less per base comparison, so frac can pass 1 -- `issued` is the "
                              "fraction of the LOP3 pipe the count phase itself occupies"}
     if cinfo["kind"] in ("screen", "direct"):
-        comparer_roof = dict(screen_roofline(cmp, n, nh), kernel="comparer", traffic=traffic)
+        per_position = committed_traffic("screen_bytes_per_position") if cinfo["kind"] == "screen" else None
+        comparer_roof = dict(screen_roofline(cmp, n, nh), kernel="comparer",
+                             traffic=per_position and round(per_position * n))
     # Finder bytes: 0.375 B of planes read per position scanned plus the 4 B
     # queue entry written per candidate; the profiled search runs each
     # finder launch alone, so its events time the kernel itself.

@@ -549,10 +549,15 @@ ScreenList screen_list(const cof_handle* h) {
 }  // namespace
 
 cof_status ensure_screen_list(cof_handle* h, uint64_t positions, bool windows) {
-  COF_CUDA(h, h->screen_items.ensure(screen_list_items(positions) * sizeof(uint4)));
+  // Both only affect the speed: where memory is short the least list will do,
+  // and the screen reads the queue window by window.
+  if (h->screen_items.ensure(screen_list_items(positions) * sizeof(uint4)) != cudaSuccess) {
+    cudaGetLastError();
+    COF_CUDA(h, h->screen_items.ensure(screen_list_items(0) * sizeof(uint4)));
+  }
   if (windows) {
     const uint64_t most = 2 * std::min<uint64_t>(kSegPositions, std::max<uint64_t>(positions, 1024));
-    COF_CUDA(h, h->screen_windows.ensure(most * sizeof(uint2)));
+    if (h->screen_windows.ensure(most * sizeof(uint2)) != cudaSuccess) cudaGetLastError();
   }
   COF_CUDA(h, h->screen_counts.ensure(screen_lists(h->sm_count) * 4));
   return COF_OK;

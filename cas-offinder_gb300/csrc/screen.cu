@@ -760,7 +760,7 @@ void run_screen(const GenomeView& g, uint32_t* queue, const uint32_t* qcount, ui
                 const ScreenGeom& geom, const ScreenTables& tb, uint32_t L, const ScreenList& list, const HitSink& sink,
                 int sm_count, cudaStream_t stream) {
   const size_t smem = (size_t)screen_entries(K) * 4;
-  const bool ready = geom.words >= kWindowWords;
+  const bool ready = geom.words >= kWindowWords && list.windows;
   auto kernel = ready ? screen_kernel<NW, K, DEG, true> : screen_kernel<NW, K, DEG, false>;
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (ready) windows_kernel<NW><<<8 * sm_count, 256, 0, stream>>>(g, queue, qcount, seg_pos0, geom.a0, L, list);

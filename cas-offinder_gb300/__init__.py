@@ -150,7 +150,7 @@ def lib():
             "cof_timer_stop": (c.c_int, [vp, c.POINTER(c.c_double)]),
             "cofx_mismatch_table": (None, [vp]),
             "cofx_bs_programs": (c.c_int, [c.c_char_p, sz, vp, vp, sz, vp, sz, vp, sz]),
-            "cofx_screen_plan": (c.c_int, [c.c_char_p, sz, c.c_int, vp, vp, sz, vp, sz]),
+            "cofx_screen_plan": (c.c_int, [c.c_char_p, sz, c.c_int, vp, vp, sz, vp, sz, u32]),
             "cofx_genome_text": (c.c_int, [c.c_char_p, vp, u64, c.POINTER(u64)]),
             "cofx_synth_record": (u64, [u64, u32, u64, c.c_double, c.c_double, u32, c.c_double, u32, u32, vp]),
         }
@@ -212,12 +212,13 @@ def bs_programs(text):
             "narrow": bool(narrow)}
 
 
-def screen_plan(text, level=-1):
-    """The table screen planned for one input file (test hook), or None where
-    none is: dict with its geometry, the records by class and `first`."""
+def screen_plan(text, level=-1, sm_count=152):
+    """The table screen planned for one input file on `sm_count` SMs (test
+    hook), or None where none is: dict with its geometry, the records by class
+    and `first`."""
     raw = text.encode() if isinstance(text, str) else bytes(text)
     info = np.zeros(27, dtype=np.uint32)
-    if lib().cofx_screen_plan(raw, len(raw), level, _ptr(info), None, 0, None, 0) != 0:
+    if lib().cofx_screen_plan(raw, len(raw), level, _ptr(info), None, 0, None, 0, sm_count) != 0:
         raise CofError(4, "parse error")
     x = [int(v) for v in info]
     if not x[0]:
@@ -226,7 +227,7 @@ def screen_plan(text, level=-1):
     out.update(L=x[1], K=x[2], a=x[3:7], q=x[7:11], base=x[11:15], cap=x[15:19])
     rec = np.zeros(out["variants"] * out["record_words"], dtype=np.uint32)
     first = np.zeros(out["words"] * (out["fields"] + 1), dtype=np.uint32)
-    lib().cofx_screen_plan(raw, len(raw), level, _ptr(info), _ptr(rec), rec.size, _ptr(first), first.size)
+    lib().cofx_screen_plan(raw, len(raw), level, _ptr(info), _ptr(rec), rec.size, _ptr(first), first.size, sm_count)
     out.update(records=rec.reshape(-1, out["record_words"]), first=first.reshape(out["words"], -1))
     return out
 

@@ -436,9 +436,9 @@ void adopt_screen(PatternGroup& g, const ScreenPlan& plan) {
     g.scan_words /= 2;
 }
 
-void build_group_host(int kind, PatternGroup& g, const std::vector<const Variant*>& vars, GroupHost& gh) {
+void build_group_host(int kind, int sm_count, PatternGroup& g, const std::vector<const Variant*>& vars, GroupHost& gh) {
   const size_t V = vars.size();
-  if (kind == 0) plan_screen(vars, g.gids, g.fpat, -1, gh.screen);
+  if (kind == 0) plan_screen(vars, g.gids, g.fpat, (uint32_t)sm_count, -1, gh.screen);
   else gh.screen = ScreenPlan();
   // A few variants may be cheaper to count at every start.
   g.direct_on = false;
@@ -671,7 +671,7 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
     cof_status ts = COF_OK;
     for (uint32_t level : g.screen_levels) {
       ScreenPlan plan;
-      plan_screen(vars, g.gids, g.fpat, (int)level, plan);
+      plan_screen(vars, g.gids, g.fpat, (uint32_t)h->sm_count, (int)level, plan);
       if (!plan.on) continue;
       float us = 1e30f;
       auto run = [&]() -> cof_status {
@@ -834,7 +834,7 @@ cof_status upload_jobs(cof_handle* h) {
                                       &PatternGroup::screen_records, &PatternGroup::screen_first,
                                       &PatternGroup::screen_tables})
         g.*b = std::move(old[gi].*b);
-    build_group_host(h->comparer_kind, g, group_vars[gi], gh[gi]);
+    build_group_host(h->comparer_kind, h->sm_count, g, group_vars[gi], gh[gi]);
     add_group(up, g, gh[gi]);
   }
   old.clear();
@@ -1866,7 +1866,7 @@ int cofx_bs_programs(const char* input, size_t len, uint32_t* info, uint32_t* pr
 }
 
 int cofx_screen_plan(const char* input, size_t len, int level, uint32_t* info, uint32_t* records, size_t records_cap,
-                     uint32_t* first, size_t first_cap) {
+                     uint32_t* first, size_t first_cap, uint32_t sm_count) {
   Job job;
   std::string err;
   if (!input || !info || !parse_job(input, len, job, err)) return 1;
@@ -1879,7 +1879,7 @@ int cofx_screen_plan(const char* input, size_t len, int level, uint32_t* info, u
   const uint32_t L = (uint32_t)job.pattern.size();
   FinderPattern pat{};
   ScreenPlan plan;
-  if (make_finder_pattern(job.pattern, revcomp(job.pattern), pat)) plan_screen(vars, gids, pat, level, plan);
+  if (make_finder_pattern(job.pattern, revcomp(job.pattern), pat)) plan_screen(vars, gids, pat, sm_count, level, plan);
   const ScreenGeom& G = plan.geom;
   uint32_t* o = info;
   for (uint32_t x : {(uint32_t)plan.on, L, G.K}) *o++ = x;

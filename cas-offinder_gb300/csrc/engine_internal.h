@@ -247,9 +247,9 @@ struct GroupHost {
   ScreenPlan screen;                 // table screen (then the others stay empty)
 };
 // Fills g's host-side fields (slots, chunks, m, screen, ...) and `gh` for
-// `vars` (ids g.gids); `kind` as cof_set_comparer.  Thread-safe: touches only
-// its arguments.
-void build_group_host(int kind, PatternGroup& g, const std::vector<const Variant*>& vars, GroupHost& gh);
+// `vars` (ids g.gids); `kind` as cof_set_comparer, `sm_count` the SMs the
+// launches get.  Thread-safe: touches only its arguments.
+void build_group_host(int kind, int sm_count, PatternGroup& g, const std::vector<const Variant*>& vars, GroupHost& gh);
 // Host-to-device copies gathered into one page-locked buffer, so that they are
 // queued without waiting.  The sources may go once `run` returns.
 struct Upload {

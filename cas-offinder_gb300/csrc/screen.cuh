@@ -39,7 +39,10 @@ constexpr uint32_t screen_run_len(uint32_t K, uint32_t k) { return K == 4 && k >
 constexpr uint32_t screen_base(uint32_t k) { return k == 0 ? 0u : k == 1 ? 16384u : k == 2 ? 32768u : 36864u; }
 constexpr uint32_t screen_entries(uint32_t K) { return K == 4 ? 40960u : 49152u; }
 constexpr uint32_t kScreenMaxLimit = 15;  // largest mismatch limit (5-bit fields)
-constexpr uint32_t kScreenMaxWords = 768;  // a CTA's share spans at most 8 of them
+// Most table words of a screen launched as `sm_count` CTAs.  A list item holds
+// its word in 3 bits, relative to the first word of its CTA's share; a share
+// of 7 words' candidates touches 8 words.
+constexpr uint32_t screen_max_words(uint32_t sm_count) { return 7 * sm_count < 768 ? 7 * sm_count : 768; }
 
 // Geometry of a group's screen (kernel argument).
 struct ScreenGeom {
@@ -71,11 +74,11 @@ struct ScreenPlan {
 };
 
 // Plans the screen of a pattern group (PAM scan `pat`) over `vars` (ids
-// `gids`).  `on` stays false where the screen cannot run (a limit above
-// 15) or its cost model puts the bit-sliced comparer ahead.  `force_level`
-// >= 0 takes that partition.
+// `gids`) for launches on `sm_count` SMs.  `on` stays false where the screen
+// cannot run (a limit above 15, more than screen_max_words) or its cost model
+// puts the bit-sliced comparer ahead.  `force_level` >= 0 takes that partition.
 void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint32_t>& gids, const FinderPattern& pat,
-                 int force_level, ScreenPlan& plan);
+                 uint32_t sm_count, int force_level, ScreenPlan& plan);
 // Text of a partition ("2/guide", "4 guides", ...).
 const char* screen_level_name(uint32_t level);
 

@@ -102,7 +102,7 @@ bool can_scan(const FinderPattern& pat, double plus, double minus) {
 }  // namespace
 
 void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint32_t>& gids, const FinderPattern& pat,
-                 int force_level, ScreenPlan& plan) {
+                 uint32_t sm_count, int force_level, ScreenPlan& plan) {
   plan = ScreenPlan();
   const size_t V = vars.size();
   const uint32_t L = pat.L;
@@ -309,7 +309,7 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
       if (force_level < 0 && lv.guides > 1 && lv.guides >= 2 * guides.size()) continue;
       if (force_level < 0 && lv.parts > 1 && V < 4 * guides.size()) continue;
       const uint32_t n = (uint32_t)((guides.size() + lv.guides - 1) / lv.guides) * lv.parts;
-      if ((n + G.fields - 1) / G.fields > kScreenMaxWords) continue;
+      if ((n + G.fields - 1) / G.fields > screen_max_words(sm_count)) continue;
       const double words = (double)((n + G.fields - 1) / G.fields), queue = queue_cost(c, words);
       double items = 0;
       const double work = c * count_work(lv, n, &items), listed = c / 2048.0 * items;

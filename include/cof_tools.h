@@ -50,16 +50,16 @@ int cofx_bs_programs(const char* input, size_t len, uint32_t* info, uint32_t* pr
                      size_t pgid_cap, char* keys, size_t keys_cap);
 
 /* Test hook: plans the table screen (cas-offinder_gb300/csrc/screen.cuh) of
- * one input file's compare variants; level < 0 lets the cost model choose the
- * partition.  info[0..26] = {planned, L, runs, first position of each run (4),
- * positions of each run (4), first entry of each run's table (4), largest
+ * one input file's compare variants for a device of `sm_count` SMs; level < 0
+ * lets the cost model choose the partition.  info[0..26] = {planned, L, runs,
+ * first position of each run (4), positions of each run (4), first entry of each run's table (4), largest
  * entry of each run's table (4), entries of a word, field bits, fields, top
  * bits, words, degenerate codes, variants, words per record}.  Each output is filled when its capacity
  * (in words) suffices: records (variants * words per record; masks t, c, a,
  * g, o and id << 4 | limit), first (words * (fields + 1)).  Returns 0, or 1
  * on a parse error. */
 int cofx_screen_plan(const char* input, size_t len, int level, uint32_t* info, uint32_t* records, size_t records_cap,
-                     uint32_t* first, size_t first_cap);
+                     uint32_t* first, size_t first_cap, uint32_t sm_count);
 
 #ifdef __cplusplus
 }

@@ -44,7 +44,7 @@ __device__ __forceinline__ uint32_t class_word(uint32_t cls, uint32_t h, uint32_
 template <int NB>
 __global__ void __launch_bounds__(kDirectThreads, kDirectCtas)
     direct_kernel(const __grid_constant__ GenomeView g, uint64_t w_begin, uint32_t words, uint64_t pos_end,
-                  const __grid_constant__ DirectParams P, uint32_t* __restrict__ qcount,
+                  const __grid_constant__ DirectParams P, unsigned long long* __restrict__ qcount,
                   const __grid_constant__ HitSink sink) {
   extern __shared__ uint32_t rows_all[];
   const unsigned lane = threadIdx.x & 31;
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(kDirectThreads, kDirectCtas)
   }
   if (qcount) {
     found = __reduce_add_sync(kFull, found);
-    if (lane == 0 && found) atomicAdd(qcount, found);
+    if (lane == 0 && found) atomicAdd(qcount, (unsigned long long)found);
   }
 }
 
@@ -210,7 +210,7 @@ double direct_cost(const DirectParams& p) {
   return c;
 }
 
-void launch_direct(const GenomeView& g, uint64_t w_begin, uint64_t w_end, const DirectParams& p, uint32_t* qcount,
+void launch_direct(const GenomeView& g, uint64_t w_begin, uint64_t w_end, const DirectParams& p, unsigned long long* qcount,
                    const HitSink& sink, int sm_count, cudaStream_t stream) {
   uint32_t most = 0;
   for (uint32_t v = 0; v < p.variants; ++v) most = std::max(most, p.n[v]);

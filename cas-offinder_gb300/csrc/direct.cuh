@@ -40,7 +40,7 @@ double direct_cost(const DirectParams& p);
 // Counts starts [32 * w_begin, 32 * w_end) below g.n - L + 1 and appends hit
 // keys; adds the candidates (starts that match the PAM, per strand) to
 // *qcount (may be null).
-void launch_direct(const GenomeView& g, uint64_t w_begin, uint64_t w_end, const DirectParams& p, uint32_t* qcount,
+void launch_direct(const GenomeView& g, uint64_t w_begin, uint64_t w_end, const DirectParams& p, unsigned long long* qcount,
                    const HitSink& sink, int sm_count, cudaStream_t stream);
 
 }  // namespace cof

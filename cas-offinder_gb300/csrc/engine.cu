@@ -578,7 +578,7 @@ void launch_group_compare(const cof_handle* h, const PatternGroup& g, uint32_t* 
                     h->sm_count, h->stream);
 }
 
-void launch_group_scan(const cof_handle* h, const PatternGroup& g, uint64_t w0, uint64_t w1, uint32_t* qc,
+void launch_group_scan(const cof_handle* h, const PatternGroup& g, uint64_t w0, uint64_t w1, unsigned long long* qc,
                        const HitSink& sink) {
   if (g.direct_on) {
     launch_direct(h->genome.view(), w0, w1, g.direct, qc, sink, h->sm_count, h->stream);
@@ -651,14 +651,15 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
     cof_status st = ensure_screen_list(h, std::min<uint64_t>(dg.n, 32 * kScanWords), true);
     if (st) return st;
   }
-  COF_CUDA(h, h->qcounts.ensure(std::max<size_t>(h->qcounts.cap, 8)));  // count, tile counter
+  COF_CUDA(h, h->qcounts.ensure(PassCounts::bytes(1)));
   COF_CUDA(h, h->hit_count.ensure(8));
   const uint64_t cap = std::max<uint64_t>(h->hits.cap / 8, 1u << 20);
   COF_CUDA(h, h->hits.ensure(cap * 8));
   const GenomeView gv = dg.view();
   uint32_t* q = h->queue[0].as<uint32_t>();
-  uint32_t* qc = h->qcounts.as<uint32_t>();
-  COF_CUDA(h, cudaMemsetAsync(qc, 0, 4, h->stream));
+  const PassCounts pc(h->qcounts, 1);
+  uint32_t* qc = pc.queue(0);
+  COF_CUDA(h, cudaMemsetAsync(qc, 0, 8, h->stream));
   if (!g.screen_on) launch_finder(gv, w0, w1, g.fpat, q, qc, h->stream);
   cudaEvent_t ev[2] = {nullptr, nullptr};
   for (cudaEvent_t& e : ev) COF_CUDA(h, cudaEventCreate(&e));
@@ -685,12 +686,12 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
         if (st) return st;
         for (int rep = 0; rep < 2; ++rep) {
           COF_CUDA(h, cudaMemsetAsync(h->hit_count.p, 0, 8, h->stream));
-          COF_CUDA(h, cudaMemsetAsync(qc, 0, 4, h->stream));
+          COF_CUDA(h, cudaMemsetAsync(qc, 0, 8, h->stream));
           COF_CUDA(h, cudaEventRecord(ev[0], h->stream));
           const ScreenTables tb{buf[0].as<uint32_t>(), buf[1].as<uint32_t>(), buf[2].as<uint32_t>()};
           const HitSink sink{h->hits.as<uint64_t>(), h->hit_count.as<unsigned long long>(), cap};
           if (plan.scans) {
-            launch_scan_screen(gv, w0, w1, g.fpat, plan.geom, tb, screen_list(h), qc, sink, h->sm_count, h->stream);
+            launch_scan_screen(gv, w0, w1, g.fpat, plan.geom, tb, screen_list(h), pc.counts, sink, h->sm_count, h->stream);
           } else {
             launch_finder(gv, w0, w1, g.fpat, q, qc, h->stream);
             launch_screen(gv, q, qc, w0 * 32, plan.geom, g.nw, tb, g.L, screen_list(h), sink, h->sm_count, h->stream);
@@ -743,10 +744,10 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
       COF_CUDA(h, cudaMemcpyAsync(dpgid.p, pgid.data(), pgid.size() * 4, cudaMemcpyHostToDevice, h->stream));
       for (int rep = 0; rep < 2; ++rep) {
         COF_CUDA(h, cudaMemsetAsync(h->hit_count.p, 0, 8, h->stream));
-        COF_CUDA(h, cudaMemsetAsync(qc + 1, 0, 4, h->stream));
+        COF_CUDA(h, cudaMemsetAsync(pc.tiles, 0, 4, h->stream));
         COF_CUDA(h, cudaEventRecord(ev[0], h->stream));
         if (!launch_comparer_bs(gv, q, qc, w0 * 32, dprog.as<uint32_t>(), dpgid.as<uint32_t>(), chunks, mm,
-                                g.bs_slots, g.bs_narrow, g.L, g.concrete_only, qc + 1, h->hits.as<uint64_t>(),
+                                g.bs_slots, g.bs_narrow, g.L, g.concrete_only, pc.tiles, h->hits.as<uint64_t>(),
                                 h->hit_count.as<unsigned long long>(), cap, h->sm_count, h->stream)) {
           declined = true;
           return COF_OK;
@@ -910,7 +911,7 @@ void collect(cof_handle* h, std::vector<EventPair>& evs) {
 // Finder + comparer over the whole genome for every pattern group; leaves the
 // hit count in h->hit_count.  Pass i = (segment s, group g) scans on stream2
 // into queue[i % 2] while the comparer works on pass i - 1 on the main
-// stream; events order the two.  qcounts[s * groups + g] keeps each pass's
+// stream; events order the two.  Pass s * groups + g of qcounts keeps its
 // candidate count.
 cof_status run_passes(cof_handle* h, uint64_t hit_cap, std::vector<EventPair>& evs, uint64_t* seg_count) {
   const DevGenome& dg = h->genome;
@@ -925,10 +926,10 @@ cof_status run_passes(cof_handle* h, uint64_t hit_cap, std::vector<EventPair>& e
   }
   const uint64_t nseg = (max_words + kSegWords - 1) / kSegWords;
   *seg_count = nseg;
-  // qcounts: candidate counts per pass, then the comparer's tile counters.
   const uint64_t nq = std::max<uint64_t>(nseg * G, 1);
-  COF_CUDA(h, h->qcounts.ensure(2 * nq * 4));
-  COF_CUDA(h, cudaMemsetAsync(h->qcounts.p, 0, 2 * nq * 4, h->stream));
+  COF_CUDA(h, h->qcounts.ensure(PassCounts::bytes(nq)));
+  COF_CUDA(h, cudaMemsetAsync(h->qcounts.p, 0, PassCounts::bytes(nq), h->stream));
+  const PassCounts pc(h->qcounts, nq);
   COF_CUDA(h, cudaMemsetAsync(h->hit_count.p, 0, 8, h->stream));
   COF_CUDA(h, cudaEventRecord(h->ev_start, h->stream));
   COF_CUDA(h, cudaStreamWaitEvent(h->stream2, h->ev_start, 0));
@@ -969,10 +970,9 @@ cof_status run_passes(cof_handle* h, uint64_t hit_cap, std::vector<EventPair>& e
         const uint64_t npos = dg.n >= g.L ? dg.n - g.L + 1 : 0;
         const uint64_t w1 = std::min((npos + 31) / 32, upto);
         if (!g.scans() || from >= w1 || g.gids.empty()) continue;
-        uint32_t* qc = h->qcounts.as<uint32_t>() + s * G + gi;
         cof_status st = record_start(h, evs, "comparer", (double)(s * G + gi), h->stream);
         if (st) return st;
-        launch_group_scan(h, g, from, w1, qc, sink);
+        launch_group_scan(h, g, from, w1, pc.counts + s * G + gi, sink);
         if ((st = record_stop(h, evs, h->stream))) return st;
       }
       from = upto;
@@ -984,7 +984,7 @@ cof_status run_passes(cof_handle* h, uint64_t hit_cap, std::vector<EventPair>& e
       const uint64_t w0 = s * kSegWords, w1 = std::min(words, w0 + kSegWords);
       if (g.scans() || w0 >= w1 || g.gids.empty()) continue;
       const int b = (int)(pass & 1);
-      uint32_t* qc = h->qcounts.as<uint32_t>() + s * G + gi;
+      uint32_t* qc = pc.queue(s * G + gi);
       uint32_t* q = h->queue[b].as<uint32_t>();
       if (pass >= 2) COF_CUDA(h, cudaStreamWaitEvent(h->stream2, h->ev_used[b], 0));
       // A profiled search times every launch alone: the finder also waits
@@ -1008,7 +1008,7 @@ cof_status run_passes(cof_handle* h, uint64_t hit_cap, std::vector<EventPair>& e
       COF_CUDA(h, cudaStreamWaitEvent(h->stream, h->ev_found[b], 0));
       // Comparer units are filled in from qcounts after the search.
       if ((st = record_start(h, evs, "comparer", (double)(s * G + gi), h->stream))) return st;
-      launch_group_compare(h, g, q, qc, qc + nq, w0 * 32, sink);
+      launch_group_compare(h, g, q, qc, pc.tiles + s * G + gi, w0 * 32, sink);
       if ((st = record_stop(h, evs, h->stream))) return st;
       COF_CUDA(h, cudaEventRecord(h->ev_used[b], h->stream));
       ++pass;
@@ -1073,7 +1073,7 @@ cof_status run_passes_graph(cof_handle* h, uint64_t cap, uint64_t* nseg) {
     max_words = std::max(max_words, (npos + 31) / 32);
   }
   const uint64_t ns = (max_words + kSegWords - 1) / kSegWords;
-  COF_CUDA(h, h->qcounts.ensure(2 * std::max<uint64_t>(ns * h->groups.size(), 1) * 4));
+  COF_CUDA(h, h->qcounts.ensure(PassCounts::bytes(std::max<uint64_t>(ns * h->groups.size(), 1))));
   const std::string key = pass_graph_key(h, cap);
   if (!h->pass_graph || key != h->pass_key) {
     if (h->pass_graph) cudaGraphExecDestroy(h->pass_graph);
@@ -1212,8 +1212,8 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
     // Comparer units: base comparisons = oriented candidates x non-N positions
     // of each variant; variant tests go to "comparer.tests".
     const size_t G = h->groups.size();
-    std::vector<uint32_t> qc(std::max<uint64_t>(nseg * G, 1), 0);
-    COF_CUDA(h, cudaMemcpy(qc.data(), h->qcounts.p, nseg * G * 4, cudaMemcpyDeviceToHost));
+    std::vector<uint64_t> qc(std::max<uint64_t>(nseg * G, 1), 0);
+    COF_CUDA(h, cudaMemcpy(qc.data(), h->qcounts.p, nseg * G * 8, cudaMemcpyDeviceToHost));
     for (EventPair& p : evs)
       if (p.name == "comparer") {
         const size_t idx = (size_t)p.units;
@@ -1223,7 +1223,7 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
         if (g.bs_slots && g.bs_chunks)  // lane LOP3 ops the bit-sliced count issues (op model)
           h->stats["comparer.lop3"].units +=
               (double)((qc[idx] + 63) / 64) * 32.0 * g.bs_chunks * bs_lane_lop3(g.bs_slots, g.bs_m, g.bs_narrow);
-        h->stats["finder.candidates"].units += (double)qc[idx];  // queue entries the finder wrote
+        h->stats["finder.candidates"].units += (double)qc[idx];
       }
     collect(h, evs);
   }

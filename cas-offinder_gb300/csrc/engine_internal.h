@@ -103,6 +103,18 @@ struct DevGenome {
   }
 };
 
+// cof_handle::qcounts for `passes` passes (segment, group): a 64-bit candidate
+// count each -- a scanning group counts a whole genome in one pass, two
+// candidates a start; a finder pass fills its queue's count, at most 2^27, in
+// the low half -- and then a 32-bit tile counter each.
+struct PassCounts {
+  unsigned long long* counts;
+  uint32_t* tiles;
+  PassCounts(const DevBuf& b, uint64_t passes) : counts(b.as<unsigned long long>()), tiles((uint32_t*)(counts + passes)) {}
+  uint32_t* queue(uint64_t pass) const { return (uint32_t*)(counts + pass); }
+  static size_t bytes(uint64_t passes) { return passes * 12; }
+};
+
 struct KernelStat {
   uint64_t launches = 0;
   double ms = 0;
@@ -273,7 +285,7 @@ void launch_group_compare(const cof_handle* h, const PatternGroup& g, uint32_t* 
                           uint32_t* tile_ctr, uint64_t pos0, const HitSink& sink);
 // Scans plane words [w0, w1) for g (scans()) on h->stream; candidates are
 // added to *qc.
-void launch_group_scan(const cof_handle* h, const PatternGroup& g, uint64_t w0, uint64_t w1, uint32_t* qc,
+void launch_group_scan(const cof_handle* h, const PatternGroup& g, uint64_t w0, uint64_t w1, unsigned long long* qc,
                        const HitSink& sink);
 // The list buffers of the screens of launches over up to `positions` starts
 // (with `windows`, those of a queue's windows too).

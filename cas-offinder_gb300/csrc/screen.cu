@@ -406,8 +406,8 @@ template <int K, bool DEG>
 __global__ void __launch_bounds__(kScanThreads, 1) scan_screen_kernel(
     const __grid_constant__ GenomeView g, uint64_t w_begin, uint32_t words, uint32_t skip, uint64_t pos_end,
     const __grid_constant__ ScanParams P, const __grid_constant__ ScreenGeom G,
-    const __grid_constant__ ScreenTables tb, const __grid_constant__ ScreenList list, uint32_t* __restrict__ qcount,
-    const __grid_constant__ HitSink sink) {
+    const __grid_constant__ ScreenTables tb, const __grid_constant__ ScreenList list,
+    unsigned long long* __restrict__ qcount, const __grid_constant__ HitSink sink) {
   extern __shared__ __align__(16) uint32_t tab[];
   __shared__ uint32_t cls[9];
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) scan_screen_kernel(
     }
     u = word_u + stop;
   }
-  if (lane == 0 && found) atomicAdd(qcount, found);
+  if (lane == 0 && found) atomicAdd(qcount, (unsigned long long)found);
   out.close(list);
 }
 
@@ -771,8 +771,8 @@ void run_screen(const GenomeView& g, uint32_t* queue, const uint32_t* qcount, ui
 
 template <int K, bool DEG>
 void run_scan_screen(const GenomeView& g, uint64_t w_begin, uint64_t w_end, const FinderPattern& pat,
-                     const ScreenGeom& geom, const ScreenTables& tb, const ScreenList& list, uint32_t* qcount,
-                     const HitSink& sink, int sm_count, cudaStream_t stream) {
+                     const ScreenGeom& geom, const ScreenTables& tb, const ScreenList& list,
+                     unsigned long long* qcount, const HitSink& sink, int sm_count, cudaStream_t stream) {
   const size_t smem = (size_t)screen_entries(K) * 4 + kScanThreads / 32 * kScanWarpBytes;
   const uint64_t pos_end = g.n >= pat.L ? g.n - pat.L + 1 : 0;
   cudaFuncSetAttribute(scan_screen_kernel<K, DEG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -821,8 +821,8 @@ void launch_screen(const GenomeView& g, uint32_t* queue, const uint32_t* qcount,
 }
 
 void launch_scan_screen(const GenomeView& g, uint64_t w_begin, uint64_t w_end, const FinderPattern& pat,
-                        const ScreenGeom& geom, const ScreenTables& tb, const ScreenList& list, uint32_t* qcount,
-                        const HitSink& sink, int sm_count, cudaStream_t stream) {
+                        const ScreenGeom& geom, const ScreenTables& tb, const ScreenList& list,
+                        unsigned long long* qcount, const HitSink& sink, int sm_count, cudaStream_t stream) {
   auto run = geom.K == 3 ? (geom.degenerate ? run_scan_screen<3, true> : run_scan_screen<3, false>)
                          : (geom.degenerate ? run_scan_screen<4, true> : run_scan_screen<4, false>);
   run(g, w_begin, w_end, pat, geom, tb, list, qcount, sink, sm_count, stream);

@@ -139,7 +139,7 @@ void launch_screen(const GenomeView& g, uint32_t* queue, const uint32_t* qcount,
 // kScanWords of them; adds the candidates found to *qcount.
 constexpr uint64_t kScanWords = 1ull << 24;
 void launch_scan_screen(const GenomeView& g, uint64_t w_begin, uint64_t w_end, const FinderPattern& pat,
-                        const ScreenGeom& geom, const ScreenTables& tb, const ScreenList& list, uint32_t* qcount,
-                        const HitSink& sink, int sm_count, cudaStream_t stream);
+                        const ScreenGeom& geom, const ScreenTables& tb, const ScreenList& list,
+                        unsigned long long* qcount, const HitSink& sink, int sm_count, cudaStream_t stream);
 
 }  // namespace cof

@@ -245,9 +245,9 @@ cof_status run_step(cof_server* s, uint64_t k) {
   uint64_t cap = std::max<uint64_t>(s->step_hits.cap / 8, 1u << 16);
   COF_CUDA(h, s->step_hits.ensure(cap * 8));
   COF_CUDA(h, s->step_count.ensure(8));
-  // candidate counts per (segment, group), then the comparer's tile counters
   const size_t nq = std::max<size_t>(T.groups.size(), 1) * (size_t)k;
-  COF_CUDA(h, h->qcounts.ensure(2 * nq * 4));
+  COF_CUDA(h, h->qcounts.ensure(PassCounts::bytes(nq)));
+  const PassCounts pc(h->qcounts, nq);
   // at most two oriented candidates per start position of a segment
   COF_CUDA(h, h->queue[0].ensure(2 * s->seg_words * 32 * 4));
   COF_CUDA(h, h->queue[1].ensure(2 * s->seg_words * 32 * 4));
@@ -256,7 +256,7 @@ cof_status run_step(cof_server* s, uint64_t k) {
   if (ls) return ls;
   uint64_t count = 0;
   for (;;) {
-    COF_CUDA(h, cudaMemsetAsync(h->qcounts.p, 0, 2 * nq * 4, h->stream));
+    COF_CUDA(h, cudaMemsetAsync(h->qcounts.p, 0, PassCounts::bytes(nq), h->stream));
     COF_CUDA(h, cudaMemsetAsync(s->step_count.p, 0, 8, h->stream));
     COF_CUDA(h, cudaEventRecord(h->ev_start, h->stream));
     COF_CUDA(h, cudaStreamWaitEvent(h->stream2, h->ev_start, 0));
@@ -271,17 +271,17 @@ cof_status run_step(cof_server* s, uint64_t k) {
       const uint64_t w0 = seg * s->seg_words, w1 = std::min(words, w0 + s->seg_words);
       if (w0 >= w1 || g.gids.empty()) continue;
       const int b = (int)(pass & 1);
-      uint32_t* qc = h->qcounts.as<uint32_t>() + si * T.groups.size() + gi;
+      const size_t at = si * T.groups.size() + gi;
       if (g.scans()) {
-        launch_group_scan(h, g, w0, w1, qc, sink);
+        launch_group_scan(h, g, w0, w1, pc.counts + at, sink);
         continue;
       }
       uint32_t* q = h->queue[b].as<uint32_t>();
       if (pass >= 2) COF_CUDA(h, cudaStreamWaitEvent(h->stream2, h->ev_used[b], 0));
-      launch_finder(gv, w0, w1, g.fpat, q, qc, h->stream2);
+      launch_finder(gv, w0, w1, g.fpat, q, pc.queue(at), h->stream2);
       COF_CUDA(h, cudaEventRecord(h->ev_found[b], h->stream2));
       COF_CUDA(h, cudaStreamWaitEvent(h->stream, h->ev_found[b], 0));
-      launch_group_compare(h, g, q, qc, qc + nq, w0 * 32, sink);
+      launch_group_compare(h, g, q, pc.queue(at), pc.tiles + at, w0 * 32, sink);
       COF_CUDA(h, cudaEventRecord(h->ev_used[b], h->stream));
       ++pass;
     }

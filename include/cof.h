@@ -359,8 +359,8 @@ cof_status cof_set_profiling(cof_handle* h, int enable);
 /* Totals since profiling was enabled for kernel `name` ("finder", "comparer",
  * "format"; "comparer.tests" counts variant tests in `units`,
  * "comparer.lop3" the lane LOP3 instructions the bit-sliced comparer's count
- * issues by its op model, "finder.candidates" the queue entries written,
- * "sort" the hit-key sort, "rows_to_host" the row copies to host memory from
+ * issues by its op model, "finder.candidates" the strand-oriented starts that
+ * match the PAM, "sort" the hit-key sort, "rows_to_host" the row copies to host memory from
  * the first chunk's copy to the last's end, `units` = bytes): launches,
  * summed device milliseconds and algorithmic units
  * (finder: genome positions scanned; comparer: base comparisons, i.e. the

@@ -44,8 +44,11 @@ EXPORTS = [
     "cof_router_open", "cof_router_add_genome", "cof_router_drop_genome", "cof_router_genomes", "cof_router_submit",
     "cof_router_wait", "cof_router_release", "cof_router_last_error", "cof_router_close",
     "cof_gzip_open", "cof_gzip_write", "cof_gzip_write_fn", "cof_gzip_close",
-    "cofx_synth_record", "cofx_mismatch_table", "cofx_bs_programs", "cofx_screen_plan", "cofx_genome_text",
+    "cofx_synth_record", "cofx_mismatch_table", "cofx_bs_programs", "cofx_screen_plan", "cofx_comparer_plan",
+    "cofx_genome_text",
 ]
+
+COMPARERS = {1: "popcount", 2: "bit-sliced", 3: "screen", 4: "direct"}
 
 # cof_write_fn: int (*)(void* ctx, const char* data, size_t len)
 WRITE_FN = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t)
@@ -151,6 +154,7 @@ def lib():
             "cofx_mismatch_table": (None, [vp]),
             "cofx_bs_programs": (c.c_int, [c.c_char_p, sz, vp, vp, sz, vp, sz, vp, sz]),
             "cofx_screen_plan": (c.c_int, [c.c_char_p, sz, c.c_int, vp, vp, sz, vp, sz, u32]),
+            "cofx_comparer_plan": (c.c_int, [c.c_char_p, sz, u64, u32, vp]),
             "cofx_genome_text": (c.c_int, [c.c_char_p, vp, u64, c.POINTER(u64)]),
             "cofx_synth_record": (u64, [u64, u32, u64, c.c_double, c.c_double, u32, c.c_double, u32, u32, vp]),
         }
@@ -230,6 +234,17 @@ def screen_plan(text, level=-1, sm_count=152):
     lib().cofx_screen_plan(raw, len(raw), level, _ptr(info), _ptr(rec), rec.size, _ptr(first), first.size, sm_count)
     out.update(records=rec.reshape(-1, out["record_words"]), first=first.reshape(out["words"], -1))
     return out
+
+
+def comparer_plan(text, positions=3_100_000_000, sm_count=152):
+    """The comparer chosen for one input file on a genome of `positions`
+    positions (test hook)."""
+    raw = text.encode() if isinstance(text, str) else bytes(text)
+    info = np.zeros(5, dtype=np.uint32)
+    if lib().cofx_comparer_plan(raw, len(raw), positions, sm_count, _ptr(info)) != 0:
+        raise CofError(4, "parse error")
+    kind, slots, words, level, scans = (int(v) for v in info)
+    return {"kind": COMPARERS[kind], "slots": slots, "words": words, "level": level, "scans": bool(scans)}
 
 
 def plane_words(n):
@@ -456,7 +471,7 @@ class CasOFFinder:
     def comparer_info(self):
         k, sl = ctypes.c_int(), ctypes.c_int()
         self._check(self._L.cof_comparer_info(self._h, ctypes.byref(k), ctypes.byref(sl)))
-        return {"kind": {1: "popcount", 2: "bit-sliced", 3: "screen", 4: "direct"}[k.value], "slots": sl.value}
+        return {"kind": COMPARERS[k.value], "slots": sl.value}
 
     # instrumentation
     def set_profiling(self, on=True):

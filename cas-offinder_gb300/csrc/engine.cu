@@ -436,16 +436,19 @@ void adopt_screen(PatternGroup& g, const ScreenPlan& plan) {
     g.scan_words /= 2;
 }
 
-void build_group_host(int kind, int sm_count, PatternGroup& g, const std::vector<const Variant*>& vars, GroupHost& gh) {
+void build_group_host(int kind, int sm_count, uint64_t positions, PatternGroup& g, const std::vector<const Variant*>& vars, GroupHost& gh) {
   const size_t V = vars.size();
   if (kind == 0) plan_screen(vars, g.gids, g.fpat, (uint32_t)sm_count, -1, gh.screen);
   else gh.screen = ScreenPlan();
+  g.screen_from = gh.screen.on ? gh.screen.from : 0;
+  if (positions < g.screen_from) gh.screen.on = false;
   // A few variants may be cheaper to count at every start.
   g.direct_on = false;
   if (kind == 0 && V >= 1 && V <= (size_t)kDirectVariants) {
     std::vector<DirectVariant> dv;
     for (size_t i = 0; i < V; ++i) dv.push_back(DirectVariant{vars[i]->key, g.gids[i], vars[i]->threshold});
-    g.direct_on = plan_direct(g.pattern, dv.data(), V, g.direct) && direct_cost(g.direct) <= gh.screen.cost;
+    g.direct_on = plan_direct(g.pattern, dv.data(), V, g.direct) &&
+                  direct_cost(g.direct) <= (gh.screen.on ? gh.screen.cost : gh.screen.counted);
     if (g.direct_on) gh.screen = ScreenPlan();
   }
   adopt_screen(g, gh.screen);
@@ -790,7 +793,12 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
 }
 
 cof_status upload_jobs(cof_handle* h) {
+  // Another genome's size may change the choice of a group's comparer.
+  const uint64_t n = h->genome.n;
+  for (const PatternGroup& g : h->groups)
+    if ((h->planned_positions < g.screen_from) != (n < g.screen_from)) h->jobs_on_device = false;
   if (h->jobs_on_device) return COF_OK;
+  h->planned_positions = n;
   // The new batch's groups take over the old one's device buffers.
   std::vector<PatternGroup> old;
   old.swap(h->groups);
@@ -835,7 +843,7 @@ cof_status upload_jobs(cof_handle* h) {
                                       &PatternGroup::screen_records, &PatternGroup::screen_first,
                                       &PatternGroup::screen_tables})
         g.*b = std::move(old[gi].*b);
-    build_group_host(h->comparer_kind, h->sm_count, g, group_vars[gi], gh[gi]);
+    build_group_host(h->comparer_kind, h->sm_count, h->genome.n, g, group_vars[gi], gh[gi]);
     add_group(up, g, gh[gi]);
   }
   old.clear();
@@ -1896,6 +1904,25 @@ int cofx_screen_plan(const char* input, size_t len, int level, uint32_t* info, u
   return 0;
 }
 
+int cofx_comparer_plan(const char* input, size_t len, uint64_t positions, uint32_t sm_count, uint32_t* info) {
+  Job job;
+  std::string err;
+  if (!input || !info || !parse_job(input, len, job, err) || job.pattern.size() > (size_t)kMaxL) return 1;
+  PatternGroup g;
+  GroupHost gh;
+  init_group(g, job.pattern);
+  std::vector<const Variant*> vars;
+  for (size_t v = 0; v < job.variants.size(); ++v) {
+    vars.push_back(&job.variants[v]);
+    g.gids.push_back((uint32_t)v);
+  }
+  build_group_host(0, (int)sm_count, positions, g, vars, gh);
+  for (uint32_t x : {(uint32_t)g.comparer(), (uint32_t)g.bs_slots, g.screen_on ? g.screen.words : 0u, g.screen_level,
+                     (uint32_t)g.screen_scans})
+    *info++ = x;
+  return 0;
+}
+
 void cofx_mismatch_table(uint8_t* out) {
   if (!out) return;
   for (int p = 0; p < 256; ++p)
@@ -1982,7 +2009,7 @@ cof_status cof_comparer_info(const cof_handle* h, int* kind, int* slots) {
   if (!h) return COF_ERR_ARG;
   int k = 0, sl = 0;
   for (const PatternGroup& g : h->groups) {
-    k = std::max(k, g.direct_on ? 4 : g.screen_on ? 3 : g.bs_slots ? 2 : 1);
+    k = std::max(k, g.comparer());
     sl = std::max(sl, g.bs_slots);
   }
   if (kind) *kind = k ? k : 1;

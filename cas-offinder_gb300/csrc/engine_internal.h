@@ -145,11 +145,13 @@ struct PatternGroup {
   std::vector<uint32_t> screen_levels;                  // partitions worth timing (cost model's best first)
   std::vector<std::pair<uint32_t, float>> screen_tuned;  // (partition, µs per segment) measured by the autotuner
   DevBuf screen_records, screen_first, screen_tables;
+  uint64_t screen_from = 0;  // the choice between screen and popcount comparer changes at this many positions (0: nowhere)
   uint64_t scan_words = kScanWords;  // words of a scanning launch: its list holds what passes
   bool screen_scans = false;  // the screen scans the planes itself: no finder pass, no candidate queue
   bool direct_on = false;     // direct count (direct.cuh): no tables, no candidates
   DirectParams direct;
   bool scans() const { return screen_scans || direct_on; }
+  int comparer() const { return direct_on ? 4 : screen_on ? 3 : bs_slots ? 2 : 1; }  // as cof_comparer_info
   // The screen extracts the queue's windows first.
   bool windows() const { return screen_on && !screen_scans && screen.words >= kWindowWords; }
   ScreenTables screen_tb() const {
@@ -189,6 +191,7 @@ struct cof_handle {
   std::vector<Job> jobs;
   std::vector<uint32_t> job_gid0;
   bool jobs_on_device = false;
+  uint64_t planned_positions = 0;  // the genome's when the groups' comparers were chosen
   int comparer_kind = 0;  // cof_set_comparer
   std::vector<PatternGroup> groups;  // jobs sharing a padded pattern share finder + comparer passes
   DevBuf vfmt, sfmt, pool;           // row formatting tables over all variants
@@ -260,8 +263,9 @@ struct GroupHost {
 };
 // Fills g's host-side fields (slots, chunks, m, screen, ...) and `gh` for
 // `vars` (ids g.gids); `kind` as cof_set_comparer, `sm_count` the SMs the
-// launches get.  Thread-safe: touches only its arguments.
-void build_group_host(int kind, int sm_count, PatternGroup& g, const std::vector<const Variant*>& vars, GroupHost& gh);
+// launches get, `positions` the genome's.  Thread-safe: touches only its
+// arguments.
+void build_group_host(int kind, int sm_count, uint64_t positions, PatternGroup& g, const std::vector<const Variant*>& vars, GroupHost& gh);
 // Host-to-device copies gathered into one page-locked buffer, so that they are
 // queued without waiting.  The sources may go once `run` returns.
 struct Upload {

@@ -65,7 +65,9 @@ struct ScreenPlan {
   bool on = false;
   bool scans = false;  // the scanning kernel rather than the finder and the screen of its queue
   double listed = 0;    // candidates expected in the list, per start
-  double cost = 1e300;  // SM clocks per 2,048 starts of the screen or, where it is ahead, the bit-sliced comparer
+  double cost = 0;          // SM clocks per 2,048 starts of the screen ...
+  double counted = 1e300;   // ... and of the comparer that runs without one
+  uint64_t from = 0;        // the screen pays for genomes of this many positions or more
   ScreenGeom geom;
   std::vector<uint32_t> records;  // screen_record_words(nw) per variant
   std::vector<uint32_t> first;    // words * (fields + 1): first record of each class of a word, then the word's end
@@ -76,7 +78,8 @@ struct ScreenPlan {
 // Plans the screen of a pattern group (PAM scan `pat`) over `vars` (ids
 // `gids`) for launches on `sm_count` SMs.  `on` stays false where the screen
 // cannot run (a limit above 15, more than screen_max_words) or its cost model
-// puts the bit-sliced comparer ahead.  `force_level` >= 0 takes that partition.
+// puts the comparer that would run without it (bit-sliced, or popcount for
+// variants of more than 32 counted positions) ahead.  `force_level` >= 0 takes that partition.
 void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint32_t>& gids, const FinderPattern& pat,
                  uint32_t sm_count, int force_level, ScreenPlan& plan);
 // Text of a partition ("2/guide", "4 guides", ...).

@@ -93,6 +93,29 @@ double queue_cost(double c, double words) {
   return finder_cost(c) + (words < kWindowWords ? words * (15.0 + 0.88 * c) : 0.3 * c + words * (15.0 + 0.65 * c));
 }
 
+// The comparer that runs where no screen does, finder included.  Bit-sliced,
+// in clocks per 32 candidates: its table build and the count (measured: 108 up
+// to 32 variants; with bulges 131 for 224 and 1,231 for 3,554; without 363 for
+// 256 and 1,250 for 1,000).  Variants of more than 32 counted positions run in
+// the popcount comparer (measured per candidate, finder included: 16 up to 32
+// variants, 30 for 96, 63 for 200 and 247 for 1,000).
+double counted_cost(double c, size_t V, bool chained, uint32_t most_positions) {
+  if (!bs_slots_for((int)most_positions)) return finder_cost(c) + c * (8.0 + 7.5 * (double)((V + 31) / 32));
+  return finder_cost(c) + c / 32 * std::max(108.0, 60.0 + (chained ? 0.36 : 1.2) * (double)V);
+}
+
+// Starts from which on a screen of cost `best` is taken instead of the popcount
+// comparer of cost `counted` (0: for any number).  Where counting the whole
+// genome takes less than 0.1 ms of 152 SMs, launches and short lists weigh more
+// than the counts: 100 40-nt NGG guides at limit 12, half the popcount
+// comparer's time on 150 Mbp (1.05 against 2.14 ms), take 68 against 62 us on
+// 3 Mbp and 41 against 26 on 100 kbp; 9 pairs of 2 x 20 nt at limit 8 take 115
+// against 322 us on 3 Mbp and 47 against 43 on 100 kbp.  There the screen runs
+// where it costs a fifth.
+uint64_t screen_from(double best, double counted) {
+  return 5.0 * best <= counted ? 0 : (uint64_t)(31.5e6 * 2048.0 / counted);
+}
+
 // The scanning kernel stages up to 320 of 2,048 starts' candidates at a time
 // and takes one-word windows.
 bool can_scan(const FinderPattern& pat, double plus, double minus) {
@@ -114,12 +137,17 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
 
   // Positions: how many variants can mismatch there.
   std::vector<uint32_t> cover(L, 0);
-  for (const Variant* v : vars)
+  uint32_t most = 0;  // positions that can mismatch, of one variant
+  for (const Variant* v : vars) {
+    uint32_t positions = 0;
     for (uint32_t k = 0; k < L; ++k) {
       const uint32_t cl = class_of(v->key[k]);
       cover[k] += cl != 0;
+      positions += cl != 0;
       if (cl > 4) G.degenerate = 1;
     }
+    most = std::max(most, positions);
+  }
   uint32_t p0 = 0, p1 = L;
   while (p0 < p1 && !cover[p0]) ++p0;
   while (p1 > p0 && !cover[p1 - 1]) --p1;
@@ -319,13 +347,11 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
       if (cost < best) best = cost, best_level = li, plan.listed = listed;
     }
     if (costs.empty()) return;
-    // The bit-sliced comparer, in clocks per 32 candidates: its table build
-    // and the count (measured: 108 up to 32 variants; with bulges 131 for 224
-    // and 1,231 for 3,554; without 363 for 256 and 1,250 for 1,000).
     const bool chained = V >= 4 * guides.size();
-    const double sliced = finder_cost(c) + c / 32 * std::max(108.0, 60.0 + (chained ? 0.36 : 1.2) * (double)V);
-    plan.cost = std::min(best, sliced);
-    if (force_level < 0 && best >= sliced) return;
+    plan.cost = best;
+    plan.counted = counted_cost(c, V, chained, most);
+    if (force_level < 0 && best >= plan.counted) return;
+    if (!bs_slots_for((int)most)) plan.from = screen_from(best, plan.counted);
     std::stable_sort(costs.begin(), costs.end());
     for (const auto& c : costs)
       if (plan.candidates.size() < 2 && c.first <= 1.8 * best) plan.candidates.push_back(c.second);

@@ -180,7 +180,7 @@ void builder_main(cof_server* s) {
     }
     ts->host.resize(ts->groups.size());
     for (size_t g = 0; g < ts->groups.size(); ++g)
-      build_group_host(s->h->comparer_kind, s->h->sm_count, ts->groups[g], vars[g], ts->host[g]);
+      build_group_host(s->h->comparer_kind, s->h->sm_count, s->h->genome.n, ts->groups[g], vars[g], ts->host[g]);
     {
       std::lock_guard<std::mutex> lock(s->mu);
       s->built = std::move(ts);

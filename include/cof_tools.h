@@ -61,6 +61,13 @@ int cofx_bs_programs(const char* input, size_t len, uint32_t* info, uint32_t* pr
 int cofx_screen_plan(const char* input, size_t len, int level, uint32_t* info, uint32_t* records, size_t records_cap,
                      uint32_t* first, size_t first_cap, uint32_t sm_count);
 
+/* Test hook: the comparer chosen for one input file's compare variants on a
+ * genome of `positions` positions and a device of `sm_count` SMs, before any
+ * timing: info[0..4] = {comparer (as cof_comparer_info), slots of the
+ * bit-sliced comparer, table words of the screen, its partition, whether it
+ * scans the planes itself}.  Returns 0, or 1 on a parse error. */
+int cofx_comparer_plan(const char* input, size_t len, uint64_t positions, uint32_t sm_count, uint32_t* info);
+
 #ifdef __cplusplus
 }
 #endif

@@ -447,8 +447,16 @@ void build_group_host(int kind, int sm_count, uint64_t positions, PatternGroup& 
   if (kind == 0 && V >= 1 && V <= (size_t)kDirectVariants) {
     std::vector<DirectVariant> dv;
     for (size_t i = 0; i < V; ++i) dv.push_back(DirectVariant{vars[i]->key, g.gids[i], vars[i]->threshold});
-    g.direct_on = plan_direct(g.pattern, dv.data(), V, g.direct) &&
-                  direct_cost(g.direct) <= (gh.screen.on ? gh.screen.cost : gh.screen.counted);
+    g.direct_on = plan_direct(g.pattern, dv.data(), V, g.direct);
+    if (g.direct_on && gh.screen.on) {
+      g.direct_on = direct_cost(g.direct) <= gh.screen.cost;
+    } else if (g.direct_on) {
+      // Only where clearly ahead: its warps take whole turns of 2,048 starts,
+      // so that its last wave may be nearly empty (8 40-nt NGG guides on 50 Mbp,
+      // even by these costs: 0.40 ms, the popcount comparer 0.31).
+      const HitCosts hits = hit_costs(vars, gh.screen);
+      g.direct_on = 1.15 * (direct_cost(g.direct) + hits.direct) <= gh.screen.counted + hits.counted;
+    }
     if (g.direct_on) gh.screen = ScreenPlan();
   }
   adopt_screen(g, gh.screen);

@@ -66,8 +66,10 @@ struct ScreenPlan {
   bool scans = false;  // the scanning kernel rather than the finder and the screen of its queue
   double listed = 0;    // candidates expected in the list, per start
   double cost = 0;          // SM clocks per 2,048 starts of the screen ...
-  double counted = 1e300;   // ... and of the comparer that runs without one
+  double counted = 0;       // ... and of the comparer that runs without one
   uint64_t from = 0;        // the screen pays for genomes of this many positions or more
+  double start_candidates = 0;  // candidates expected per 2,048 starts
+  uint32_t most = 0;            // positions that can mismatch, of one variant
   ScreenGeom geom;
   std::vector<uint32_t> records;  // screen_record_words(nw) per variant
   std::vector<uint32_t> first;    // words * (fields + 1): first record of each class of a word, then the word's end
@@ -82,6 +84,13 @@ struct ScreenPlan {
 // variants of more than 32 counted positions) ahead.  `force_level` >= 0 takes that partition.
 void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint32_t>& gids, const FinderPattern& pat,
                  uint32_t sm_count, int force_level, ScreenPlan& plan);
+// What writing the hits that random windows give adds to the direct count and
+// to the comparer that runs without a screen, in clocks per 2,048 starts, for
+// a few variants; `plan` as plan_screen left it.
+struct HitCosts {
+  double direct, counted;
+};
+HitCosts hit_costs(const std::vector<const Variant*>& vars, const ScreenPlan& plan);
 // Text of a partition ("2/guide", "4 guides", ...).
 const char* screen_level_name(uint32_t level);
 

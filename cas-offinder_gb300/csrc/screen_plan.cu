@@ -130,15 +130,14 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
   const size_t V = vars.size();
   const uint32_t L = pat.L;
   if (V == 0 || L == 0 || L > (uint32_t)kMaxL) return;
-  uint32_t limit = 0;
-  for (const Variant* v : vars) limit = std::max<uint32_t>(limit, v->threshold);
-  if (limit > kScreenMaxLimit) return;
   ScreenGeom& G = plan.geom;
+  uint32_t limit = 0;
 
   // Positions: how many variants can mismatch there.
   std::vector<uint32_t> cover(L, 0);
   uint32_t most = 0;  // positions that can mismatch, of one variant
   for (const Variant* v : vars) {
+    limit = std::max<uint32_t>(limit, v->threshold);
     uint32_t positions = 0;
     for (uint32_t k = 0; k < L; ++k) {
       const uint32_t cl = class_of(v->key[k]);
@@ -148,6 +147,17 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
     }
     most = std::max(most, positions);
   }
+  // Share of random windows that match the PAM, per strand.
+  double share[2] = {1.0, 1.0};
+  for (uint32_t st = 0; st < 2; ++st)
+    for (uint32_t j = 0; j < (st ? pat.nr : pat.nf); ++j)
+      share[st] *= (4 - __builtin_popcount((st ? pat.rm[j] : pat.fm[j]) & 15u)) / 4.0;
+  const double c = (share[0] + share[1]) * 2048.0;
+  const bool may_scan = can_scan(pat, share[0], share[1]);
+  plan.counted = counted_cost(c, V, false, most);  // also where no screen can run
+  plan.start_candidates = c;
+  plan.most = most;
+  if (limit > kScreenMaxLimit) return;
   uint32_t p0 = 0, p1 = L;
   while (p0 < p1 && !cover[p0]) ++p0;
   while (p1 > p0 && !cover[p1 - 1]) --p1;
@@ -320,13 +330,6 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
       *items = q * words;
       return words * (0.5 * (1.0 - std::pow(1.0 - q, 32.0)) + 4.3 * q) + 3.4 * counts / classes * n;
     };
-    // Share of random windows that match the PAM, per strand.
-    double share[2] = {1.0, 1.0};
-    for (uint32_t st = 0; st < 2; ++st)
-      for (uint32_t j = 0; j < (st ? pat.nr : pat.nf); ++j)
-        share[st] *= (4 - __builtin_popcount((st ? pat.rm[j] : pat.fm[j]) & 15u)) / 4.0;
-    const double c = (share[0] + share[1]) * 2048.0;
-    const bool may_scan = can_scan(pat, share[0], share[1]);
     double best = 1e300;
     uint32_t best_level = 0;
     std::vector<std::pair<double, uint32_t>> costs;
@@ -391,6 +394,41 @@ void plan_screen(const std::vector<const Variant*>& vars, const std::vector<uint
     }
   }
   plan.on = true;
+}
+
+// The comparers write a 32-candidate group's hits one candidate after the
+// other, so that the bit-sliced one waits for the variant with the most
+// (measured: 210 clocks a turn) and the popcount one for each candidate with
+// some (190).  The direct count writes the hits of a word of 32 starts one
+// after the other, a warp's 32 words in step: 47 clocks a turn and 15 a hit
+// (8 40-nt NGG guides at limit 24, 24 hits in 1,000 windows: 6,665 clocks
+// measured, 6,743 by this sum; one at limit 40, all windows hits: 5,615 and
+// 5,583).
+HitCosts hit_costs(const std::vector<const Variant*>& vars, const ScreenPlan& plan) {
+  const double c = plan.start_candidates;
+  double none = 1.0, top = 0.0, direct = 0.0;
+  for (const Variant* v : vars) {
+    // P[a random window has at most the limit's mismatches].
+    std::vector<double> mm(1, 1.0);
+    for (char ch : v->key) {
+      const double q = __builtin_popcount(class_bits_of((unsigned char)ch) & 15u) / 4.0;
+      if (q == 0) continue;
+      mm.push_back(0.0);
+      for (size_t k = mm.size() - 1; k; --k) mm[k] = mm[k] * (1 - q) + mm[k - 1] * q;
+      mm[0] *= 1 - q;
+    }
+    double p = 0;
+    for (size_t k = 0; k < mm.size() && k <= v->threshold; ++k) p += mm[k];
+    none *= 1 - std::min(p, 1.0);
+    top = std::max(top, p);
+    const double word = c * p / 128;  // hits expected of 32 starts on one strand
+    const double turns = std::min(32.0, std::min(1.0, 32 * word) * (word + 2.07 * std::sqrt(word) + 0.7));
+    direct += 4 * 47.0 * turns + 15.0 * c * p;
+  }
+  if (!bs_slots_for((int)plan.most)) return HitCosts{direct, 190.0 * c * (1 - none)};
+  // The largest of V binomials of 32 candidates.
+  const double spread = std::sqrt(std::log((double)vars.size()) * 32 * top * (1 - std::min(top, 1.0)));
+  return HitCosts{direct, 210.0 * c / 32 * std::min(32.0, 32 * top + spread)};
 }
 
 }  // namespace cof

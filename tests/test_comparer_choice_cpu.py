@@ -31,6 +31,26 @@ def test_long_patterns_compare_with_the_popcount_comparer(P, built, spec, kind):
     assert P.comparer_plan(text(*spec), 30_000_000)["kind"] == kind
 
 
+# Up to 8 variants the direct count is compared with the comparer that runs
+# where no screen can (limits above 15, spellings of fewer than 9 positions;
+# ms on 50 Mbp, direct / counted).
+@pytest.mark.parametrize("spec, kind", [
+    (((32,), "NNGRRT", 8, 16), "bit-sliced"),  # 0.338 / 0.063
+    (((25,), "NNAGAAW", 8, 16), "bit-sliced"),  # 0.283 / 0.069
+    (((8,), "NNGRRT", 8, 1), "bit-sliced"),  # 0.111 / 0.050
+    (((28,), "NGG", 8, 16), "bit-sliced"),  # 0.546 / 0.363
+    (((40,), "NNGRRT", 8, 16), "popcount"),  # 0.406 / 0.109
+    (((40,), "NGG", 8, 20), "popcount"),  # 0.404 / 0.321
+    (((40,), "NGG", 4, 20), "direct"),  # 0.211 / 0.316
+    (((8,), "NGG", 1, 1), "direct"),  # 0.031 / 0.100
+    (((21,), "NNGRRT", 1, 16), "direct"),  # 0.133 / 0.711: two of three candidates are hits
+    (((20,), "NGG", 8, 16), "direct"),  # 2.77 / 3.75
+    (((20, 20), "", 8, 16), "direct"),
+])
+def test_direct_count_is_compared_where_no_screen_can_run(P, built, spec, kind):
+    assert P.comparer_plan(text(*spec))["kind"] == kind
+
+
 # Where the whole count is short, only a screen far ahead is taken.
 @pytest.mark.parametrize("spec, kind", [
     (((40,), "NGG", 100, 12), "popcount"),  # 41 / 26 us on 100 kbp

@@ -657,11 +657,22 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
   const uint64_t words = (npos + 31) / 32;
   if (words < 2 * kSegWords) return COF_OK;
   const uint64_t w0 = (words / kSegWords / 2) * kSegWords, w1 = std::min(words, w0 + kSegWords);
-  if (!g.screen_scans || g.screen_levels.size() > 1) COF_CUDA(h, h->queue[0].ensure(2 * kSegPositions * 4));
+  // The screen's partitions to time, and what they run on.
+  std::vector<ScreenPlan> plans;
+  bool queued = !g.screen_on, windows = false;
   if (g.screen_on) {
-    cof_status st = ensure_screen_list(h, std::min<uint64_t>(dg.n, 32 * kScanWords), true);
+    for (uint32_t level : g.screen_levels) {
+      ScreenPlan plan;
+      plan_screen(vars, g.gids, g.fpat, (uint32_t)h->sm_count, (int)level, plan);
+      if (!plan.on) continue;
+      queued |= !plan.scans;
+      windows |= plan.windows();
+      plans.push_back(std::move(plan));
+    }
+    cof_status st = ensure_screen_list(h, std::min<uint64_t>(dg.n, 32 * kScanWords), windows);
     if (st) return st;
   }
+  if (queued) COF_CUDA(h, h->queue[0].ensure(2 * kSegPositions * 4));
   COF_CUDA(h, h->qcounts.ensure(PassCounts::bytes(1)));
   COF_CUDA(h, h->hit_count.ensure(8));
   const uint64_t cap = std::max<uint64_t>(h->hits.cap / 8, 1u << 20);
@@ -681,10 +692,7 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
     ScreenPlan best_plan;
     DevBuf(&buf)[3] = h->tune_bufs;
     cof_status ts = COF_OK;
-    for (uint32_t level : g.screen_levels) {
-      ScreenPlan plan;
-      plan_screen(vars, g.gids, g.fpat, (uint32_t)h->sm_count, (int)level, plan);
-      if (!plan.on) continue;
+    for (ScreenPlan& plan : plans) {
       float us = 1e30f;
       auto run = [&]() -> cof_status {
         COF_CUDA(h, buf[0].ensure(plan.records.size() * 4));
@@ -717,7 +725,7 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
         return COF_OK;
       };
       if ((ts = run())) break;
-      g.screen_tuned.emplace_back(level, us);
+      g.screen_tuned.emplace_back(plan.level, us);
       if (us < best_us) {
         best_us = us;
         best_plan = std::move(plan);

@@ -75,6 +75,7 @@ struct ScreenPlan {
   std::vector<uint32_t> first;    // words * (fields + 1): first record of each class of a word, then the word's end
   uint32_t level = 0;             // the partition taken (index of screen_levels)
   std::vector<uint32_t> candidates;  // levels worth timing, the model's best first
+  bool windows() const;  // it extracts the queue's windows first
 };
 
 // Plans the screen of a pattern group (PAM scan `pat`) over `vars` (ids
@@ -110,6 +111,7 @@ struct ScreenList {
 // Words from which on a queue's windows are extracted once, ahead of the
 // lookups (measured: a gain at 16, none at 4).
 constexpr uint32_t kWindowWords = 8;
+inline bool ScreenPlan::windows() const { return on && !scans && geom.words >= kWindowWords; }
 // Set in an item whose window may hold a non-base byte (a bit that is neither
 // a field's top bit nor part of the relative word).
 constexpr uint32_t kOddWindow = 1u << 5;

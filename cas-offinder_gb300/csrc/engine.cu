@@ -123,6 +123,7 @@ cof_status upload_genome(cof_handle* h, DevGenome& dg, const uint32_t* hi, const
                          bool streamed = false) {
   const uint64_t W = plane_words(n);
   dg.loaded = false;
+  if (!streamed) h->memory_short = false;
   // The record table must describe the genome like the reference's m_chrpos:
   // first start 0, non-decreasing, inside the genome.
   if (n >= (1ull << 36)) return fail(h, COF_ERR_UNSUPPORTED, "genome longer than 2^36 positions");
@@ -138,9 +139,9 @@ cof_status upload_genome(cof_handle* h, DevGenome& dg, const uint32_t* hi, const
     if (starts[i] == 0 || !(ot[w] & b) || !(lo[w] & b) || (hi[w] & b))
       return fail(h, COF_ERR_ARG, "no ';' separator before record " + std::to_string(i) + " in the planes");
   }
-  COF_CUDA(h, dg.hi.ensure(W * 4));
-  COF_CUDA(h, dg.lo.ensure(W * 4));
-  COF_CUDA(h, dg.ot.ensure(W * 4));
+  COF_CUDA(h, need(h, dg.hi, W * 4));
+  COF_CUDA(h, need(h, dg.lo, W * 4));
+  COF_CUDA(h, need(h, dg.ot, W * 4));
   h->upload_pending = 0;
   if (!streamed) {
     COF_CUDA(h, cudaMemcpyAsync(dg.hi.p, hi, W * 4, cudaMemcpyHostToDevice, h->stream));
@@ -155,8 +156,8 @@ cof_status upload_genome(cof_handle* h, DevGenome& dg, const uint32_t* hi, const
     h->upload_issued = 0;
     h->upload_pending = chunks;
   }
-  COF_CUDA(h, dg.exc_pos.ensure(n_exc * 8));
-  COF_CUDA(h, dg.exc_byte.ensure(n_exc));
+  COF_CUDA(h, need(h, dg.exc_pos, n_exc * 8));
+  COF_CUDA(h, need(h, dg.exc_byte, n_exc));
   if (n_exc) {
     COF_CUDA(h, cudaMemcpyAsync(dg.exc_pos.p, exc_pos, n_exc * 8, cudaMemcpyHostToDevice, h->stream));
     COF_CUDA(h, cudaMemcpyAsync(dg.exc_byte.p, exc_byte, n_exc, cudaMemcpyHostToDevice, h->stream));
@@ -502,7 +503,7 @@ void build_group_host(int kind, int sm_count, uint64_t positions, PatternGroup& 
 // Fills a planned screen's tables on `st`, behind the copies of its records.
 cof_status fill_screen(cof_handle* h, const ScreenPlan& plan, int nw, DevBuf& records, DevBuf& first, DevBuf& tables,
                        cudaStream_t st) {
-  COF_CUDA(h, tables.ensure((size_t)plan.geom.words * screen_entries(plan.geom.K) * 4));
+  COF_CUDA(h, need(h, tables, (size_t)plan.geom.words * screen_entries(plan.geom.K) * 4));
   launch_screen_tables(plan.geom, nw, records.as<uint32_t>(), first.as<uint32_t>(), tables.as<uint32_t>(), st);
   COF_CUDA(h, cudaGetLastError());
   return COF_OK;
@@ -527,7 +528,7 @@ cof_status upload_group(cof_handle* h, PatternGroup& g, const GroupHost& gh, cud
   Upload up;
   add_group(up, g, gh);
   for (const Upload::Part& p : up.parts) {
-    COF_CUDA(h, p.dst->ensure(std::max<size_t>(p.bytes, 1)));
+    COF_CUDA(h, need(h, *p.dst, std::max<size_t>(p.bytes, 1)));
     COF_CUDA(h, cudaMemcpyAsync(p.dst->p, p.src, p.bytes, cudaMemcpyHostToDevice, st));
   }
   return g.screen_on ? fill_screen(h, gh.screen, g.nw, g.screen_records, g.screen_first, g.screen_tables, st) : COF_OK;
@@ -539,7 +540,7 @@ cof_status Upload::run(cof_handle* h, HostPinned& stage, cudaStream_t st) {
   COF_CUDA(h, stage.ensure(total));
   char* at = (char*)stage.p;
   for (const Part& p : parts) {
-    COF_CUDA(h, p.dst->ensure(std::max<size_t>(p.bytes, 1)));
+    COF_CUDA(h, need(h, *p.dst, std::max<size_t>(p.bytes, 1)));
     if (!p.bytes) continue;
     std::memcpy(at, p.src, p.bytes);
     COF_CUDA(h, cudaMemcpyAsync(p.dst->p, at, p.bytes, cudaMemcpyHostToDevice, st));
@@ -559,18 +560,42 @@ ScreenList screen_list(const cof_handle* h) {
 }
 }  // namespace
 
+cudaError_t need(cof_handle* h, DevBuf& b, size_t bytes) {
+  cudaError_t e = b.ensure(bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  if (give_back(h) && (e = b.ensure(bytes)) == cudaErrorMemoryAllocation) cudaGetLastError();
+  return e;
+}
+
+bool give_back(cof_handle* h) {
+  if (!h->screen_items.p && !h->screen_windows.p) return false;
+  h->screen_items.release();
+  h->screen_windows.release();
+  h->memory_short = true;
+  return true;
+}
+
 cof_status ensure_screen_list(cof_handle* h, uint64_t positions, bool windows) {
-  // Both only affect the speed: where memory is short the least list will do,
-  // and the screen reads the queue window by window.
-  if (h->screen_items.ensure(screen_list_items(positions) * sizeof(uint4)) != cudaSuccess) {
+  // Both only affect the speed: where memory is short a screen makes do with
+  // the list it had, the least one or none, and reads the queue window by
+  // window.
+  auto take = [](DevBuf& b, size_t bytes) {
+    if (b.ensure(bytes) == cudaSuccess) return true;
     cudaGetLastError();
-    COF_CUDA(h, h->screen_items.ensure(screen_list_items(0) * sizeof(uint4)));
+    return false;
+  };
+  const size_t keep = std::max(h->screen_items.cap, (size_t)screen_list_items(0) * sizeof(uint4));
+  if (!take(h->screen_items, h->memory_short ? keep : (size_t)screen_list_items(positions) * sizeof(uint4))) {
+    h->memory_short = true;
+    if (!take(h->screen_items, keep)) take(h->screen_items, screen_list_items(0) * sizeof(uint4));
   }
-  if (windows) {
-    const uint64_t most = 2 * std::min<uint64_t>(kSegPositions, std::max<uint64_t>(positions, 1024));
-    if (h->screen_windows.ensure(most * sizeof(uint2)) != cudaSuccess) cudaGetLastError();
+  const size_t most = 2 * std::min<uint64_t>(kSegPositions, std::max<uint64_t>(positions, 1024)) * sizeof(uint2);
+  if (windows && h->screen_windows.cap < most && (h->memory_short || !take(h->screen_windows, most))) {
+    h->memory_short = true;
+    h->screen_windows.release();  // one too short for the queue
   }
-  COF_CUDA(h, h->screen_counts.ensure(screen_lists(h->sm_count) * 4));
+  COF_CUDA(h, need(h, h->screen_counts, screen_lists(h->sm_count) * 4));
   return COF_OK;
 }
 
@@ -669,14 +694,16 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
       windows |= plan.windows();
       plans.push_back(std::move(plan));
     }
+  }
+  if (queued) COF_CUDA(h, need(h, h->queue[0], 2 * kSegPositions * 4));
+  COF_CUDA(h, need(h, h->qcounts, PassCounts::bytes(1)));
+  COF_CUDA(h, need(h, h->hit_count, 8));
+  const uint64_t cap = std::max<uint64_t>(h->hits.cap / 8, 1u << 20);
+  COF_CUDA(h, need(h, h->hits, cap * 8));
+  if (g.screen_on) {
     cof_status st = ensure_screen_list(h, std::min<uint64_t>(dg.n, 32 * kScanWords), windows);
     if (st) return st;
   }
-  if (queued) COF_CUDA(h, h->queue[0].ensure(2 * kSegPositions * 4));
-  COF_CUDA(h, h->qcounts.ensure(PassCounts::bytes(1)));
-  COF_CUDA(h, h->hit_count.ensure(8));
-  const uint64_t cap = std::max<uint64_t>(h->hits.cap / 8, 1u << 20);
-  COF_CUDA(h, h->hits.ensure(cap * 8));
   const GenomeView gv = dg.view();
   uint32_t* q = h->queue[0].as<uint32_t>();
   const PassCounts pc(h->qcounts, 1);
@@ -695,8 +722,8 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
     for (ScreenPlan& plan : plans) {
       float us = 1e30f;
       auto run = [&]() -> cof_status {
-        COF_CUDA(h, buf[0].ensure(plan.records.size() * 4));
-        COF_CUDA(h, buf[1].ensure(plan.first.size() * 4));
+        COF_CUDA(h, need(h, buf[0], plan.records.size() * 4));
+        COF_CUDA(h, need(h, buf[1], plan.first.size() * 4));
         COF_CUDA(h, cudaMemcpyAsync(buf[0].p, plan.records.data(), plan.records.size() * 4, cudaMemcpyHostToDevice,
                                     h->stream));
         COF_CUDA(h, cudaMemcpyAsync(buf[1].p, plan.first.data(), plan.first.size() * 4, cudaMemcpyHostToDevice,
@@ -757,8 +784,8 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
     float us = 1e30f;
     bool declined = false;  // the launcher refused this geometry: m is not a candidate
     auto run = [&]() -> cof_status {
-      COF_CUDA(h, dprog.ensure(prog.size() * 4));
-      COF_CUDA(h, dpgid.ensure(pgid.size() * 4));
+      COF_CUDA(h, need(h, dprog, prog.size() * 4));
+      COF_CUDA(h, need(h, dpgid, pgid.size() * 4));
       COF_CUDA(h, cudaMemcpyAsync(dprog.p, prog.data(), prog.size() * 4, cudaMemcpyHostToDevice, h->stream));
       COF_CUDA(h, cudaMemcpyAsync(dpgid.p, pgid.data(), pgid.size() * 4, cudaMemcpyHostToDevice, h->stream));
       for (int rep = 0; rep < 2; ++rep) {
@@ -795,8 +822,8 @@ cof_status autotune_group(cof_handle* h, PatternGroup& g, const std::vector<cons
     if (e) cudaEventDestroy(e);
   if (st) return st;
   if (best_m != g.bs_m) {
-    COF_CUDA(h, g.bs_prog.ensure(best_prog.size() * 4));
-    COF_CUDA(h, g.bs_pgid.ensure(best_pgid.size() * 4));
+    COF_CUDA(h, need(h, g.bs_prog, best_prog.size() * 4));
+    COF_CUDA(h, need(h, g.bs_pgid, best_pgid.size() * 4));
     COF_CUDA(h, cudaMemcpyAsync(g.bs_prog.p, best_prog.data(), best_prog.size() * 4, cudaMemcpyHostToDevice,
                                 h->stream));
     COF_CUDA(h, cudaMemcpyAsync(g.bs_pgid.p, best_pgid.data(), best_pgid.size() * 4, cudaMemcpyHostToDevice,
@@ -951,7 +978,7 @@ cof_status run_passes(cof_handle* h, uint64_t hit_cap, std::vector<EventPair>& e
   const uint64_t nseg = (max_words + kSegWords - 1) / kSegWords;
   *seg_count = nseg;
   const uint64_t nq = std::max<uint64_t>(nseg * G, 1);
-  COF_CUDA(h, h->qcounts.ensure(PassCounts::bytes(nq)));
+  COF_CUDA(h, need(h, h->qcounts, PassCounts::bytes(nq)));
   COF_CUDA(h, cudaMemsetAsync(h->qcounts.p, 0, PassCounts::bytes(nq), h->stream));
   const PassCounts pc(h->qcounts, nq);
   COF_CUDA(h, cudaMemsetAsync(h->hit_count.p, 0, 8, h->stream));
@@ -1097,7 +1124,7 @@ cof_status run_passes_graph(cof_handle* h, uint64_t cap, uint64_t* nseg) {
     max_words = std::max(max_words, (npos + 31) / 32);
   }
   const uint64_t ns = (max_words + kSegWords - 1) / kSegWords;
-  COF_CUDA(h, h->qcounts.ensure(PassCounts::bytes(std::max<uint64_t>(ns * h->groups.size(), 1))));
+  COF_CUDA(h, need(h, h->qcounts, PassCounts::bytes(std::max<uint64_t>(ns * h->groups.size(), 1))));
   const std::string key = pass_graph_key(h, cap);
   if (!h->pass_graph || key != h->pass_key) {
     if (h->pass_graph) cudaGraphExecDestroy(h->pass_graph);
@@ -1143,7 +1170,7 @@ cof_status summarise(cof_handle* h, uint64_t nhits) {
     for (const Variant& v : job.variants) levels = std::max<uint32_t>(levels, (uint32_t)v.threshold + 1);
   levels = std::min<uint32_t>(levels, 128);
   const size_t ncount = (size_t)G * 2 * levels;
-  COF_CUDA(h, h->summary_counts.ensure(ncount * 4));
+  COF_CUDA(h, need(h, h->summary_counts, ncount * 4));
   COF_CUDA(h, cudaMemsetAsync(h->summary_counts.p, 0, ncount * 4, h->stream));
   launch_hit_histogram(h->hits_sorted.as<uint64_t>(), nhits, levels, h->summary_counts.as<uint32_t>(), h->stream);
   COF_CUDA(h, cudaGetLastError());
@@ -1187,11 +1214,10 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
     windows |= g.windows();
   }
   if (queues)
-    for (DevBuf& q : h->queue) COF_CUDA(h, q.ensure(2 * kSegPositions * 4));
-  if (screens && (st = ensure_screen_list(h, std::min<uint64_t>(h->genome.n, 32 * kScanWords), windows))) return st;
-  COF_CUDA(h, h->hit_count.ensure(8));
+    for (DevBuf& q : h->queue) COF_CUDA(h, need(h, q, 2 * kSegPositions * 4));
+  COF_CUDA(h, need(h, h->hit_count, 8));
   uint64_t cap = std::max<uint64_t>(h->hits.cap / 8, 1u << 20);
-  COF_CUDA(h, h->hits.ensure(cap * 8));
+  COF_CUDA(h, need(h, h->hits, cap * 8));
   std::vector<EventPair> evs;
   uint64_t nseg = 0, nhits = 0;
   // Profiled searches time each launch with events, and those under a streamed
@@ -1204,12 +1230,13 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
   constexpr uint64_t kSmallText = 1ull << 20;
   const bool small = !h->profiling && J <= kSmallJobs;
   if (small) {
-    for (DevBuf* b : {&h->hits_sorted, &h->row_offsets, &h->row_bytes}) COF_CUDA(h, b->ensure(kSmallHits * 8));
+    for (DevBuf* b : {&h->hits_sorted, &h->row_offsets, &h->row_bytes}) COF_CUDA(h, need(h, *b, kSmallHits * 8));
     COF_CUDA(h, h->small_out.ensure(sizeof(SmallOut)));
     COF_CUDA(h, h->host_text.ensure(kSmallText + 1));
   }
   const SmallOut* so = (const SmallOut*)h->small_out.p;
   for (;;) {
+    if (screens && (st = ensure_screen_list(h, std::min<uint64_t>(h->genome.n, 32 * kScanWords), windows))) return st;
     st = graph ? run_passes_graph(h, cap, &nseg) : run_passes(h, cap, evs, &nseg);
     if (st) return st;
     if (small) {
@@ -1230,7 +1257,7 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
     }
     evs.clear();
     cap = nhits + nhits / 8;
-    COF_CUDA(h, h->hits.ensure(cap * 8));
+    COF_CUDA(h, need(h, h->hits, cap * 8));
   }
   if (h->profiling) {
     // Comparer units: base comparisons = oriented candidates x non-N positions
@@ -1268,12 +1295,12 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
     return h->summary_on ? summarise(h, nhits) : COF_OK;
   }
   // Sort hit keys into output order.
-  COF_CUDA(h, h->hits_sorted.ensure(nhits * 8));
-  COF_CUDA(h, h->row_bytes.ensure(nhits * 8));
-  COF_CUDA(h, h->row_offsets.ensure(nhits * 8));
-  COF_CUDA(h, h->row_count.ensure(nhits * 4));
-  COF_CUDA(h, h->small.ensure(64));
-  COF_CUDA(h, h->job_bytes.ensure((J + 1) * 8));
+  COF_CUDA(h, need(h, h->hits_sorted, nhits * 8));
+  COF_CUDA(h, need(h, h->row_bytes, nhits * 8));
+  COF_CUDA(h, need(h, h->row_offsets, nhits * 8));
+  COF_CUDA(h, need(h, h->row_count, nhits * 4));
+  COF_CUDA(h, need(h, h->small, 64));
+  COF_CUDA(h, need(h, h->job_bytes, (J + 1) * 8));
   // Key bits the order depends on: strand (bit 7), position, variant id up to
   // the largest id in use.  The mismatch bits below never break a tie: a
   // (variant, position, strand) has one hit at most.
@@ -1289,7 +1316,7 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
   size_t tmp3 = 0;
   COF_CUDA(h, cub::DeviceReduce::Sum(nullptr, tmp3, h->row_count.as<uint32_t>(), h->small.as<uint64_t>(),
                                      (int64_t)nhits, h->stream));
-  COF_CUDA(h, h->sort_tmp.ensure(std::max(tmp, std::max(tmp2, tmp3))));
+  COF_CUDA(h, need(h, h->sort_tmp, std::max(tmp, std::max(tmp2, tmp3))));
   tmp = h->sort_tmp.cap;
   if ((st = record_start(h, evs, "sort", (double)nhits, h->stream))) return st;
   COF_CUDA(h, cub::DeviceRadixSort::SortKeys(h->sort_tmp.p, tmp, h->hits.as<uint64_t>(), h->hits_sorted.as<uint64_t>(),
@@ -1337,7 +1364,7 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
   if (!sink) {
     // Chunk k's rows are copied to the host on the second stream (idle once
     // the passes have joined) while chunk k + 1 is written.
-    COF_CUDA(h, h->text.ensure(bytes + 1));
+    COF_CUDA(h, need(h, h->text, bytes + 1));
     COF_CUDA(h, h->host_text.ensure(bytes + 1));
     if (!h->stream_ev[0]) COF_CUDA(h, cudaEventCreateWithFlags(&h->stream_ev[0], cudaEventDisableTiming));
     ck[0] = 0;
@@ -1389,7 +1416,7 @@ cof_status do_search(cof_handle* h, const char** rows, size_t* rows_len, StreamS
     uint64_t most = 0;
     for (uint64_t k = 0; k < nb; ++k) most = std::max(most, cut[k + 1] - cut[k]);
     for (int b = 0; b < 2; ++b) {
-      COF_CUDA(h, h->stream_dev[b].ensure(most + 16));
+      COF_CUDA(h, need(h, h->stream_dev[b], most + 16));
       COF_CUDA(h, h->stream_host[b].ensure(most + 16));
       if (!h->stream_ev[b]) COF_CUDA(h, cudaEventCreateWithFlags(&h->stream_ev[b], cudaEventDisableTiming));
     }
@@ -1755,8 +1782,8 @@ cof_status cof_finder_chunk(cof_handle* h, const char* chr, uint64_t worksize, c
   make_finder_pattern(std::string(pat, patternlen), std::string(pat + patternlen, patternlen), fp);
   const uint64_t words = (worksize + 31) / 32;
   DevBuf q, qc;
-  COF_CUDA(h, q.ensure(words * 64 * 4));
-  COF_CUDA(h, qc.ensure(4));
+  COF_CUDA(h, need(h, q, words * 64 * 4));
+  COF_CUDA(h, need(h, qc, 4));
   COF_CUDA(h, cudaMemsetAsync(qc.p, 0, 4, h->stream));
   launch_finder(h->scratch.view(), 0, words, fp, q.as<uint32_t>(), qc.as<uint32_t>(), h->stream);
   COF_CUDA(h, cudaGetLastError());
@@ -1820,11 +1847,11 @@ cof_status cof_comparer_chunk(cof_handle* h, const char* chr, uint64_t chrlen, c
   else fill_mask<2>(*(VariantMask<2>*)vm.data(), cs, threshold, 0);
   DevBuf q, qc, vmd, hb, hc;
   const uint64_t cap = entries.size();
-  COF_CUDA(h, q.ensure(entries.size() * 4));
-  COF_CUDA(h, qc.ensure(4));
-  COF_CUDA(h, vmd.ensure(vm.size()));
-  COF_CUDA(h, hb.ensure(cap * 8));
-  COF_CUDA(h, hc.ensure(8));
+  COF_CUDA(h, need(h, q, entries.size() * 4));
+  COF_CUDA(h, need(h, qc, 4));
+  COF_CUDA(h, need(h, vmd, vm.size()));
+  COF_CUDA(h, need(h, hb, cap * 8));
+  COF_CUDA(h, need(h, hc, 8));
   const uint32_t ne = (uint32_t)entries.size();
   COF_CUDA(h, cudaMemcpyAsync(q.p, entries.data(), entries.size() * 4, cudaMemcpyHostToDevice, h->stream));
   COF_CUDA(h, cudaMemcpyAsync(qc.p, &ne, 4, cudaMemcpyHostToDevice, h->stream));

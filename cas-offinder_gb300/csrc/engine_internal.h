@@ -197,6 +197,10 @@ struct cof_handle {
   DevBuf vfmt, sfmt, pool;           // row formatting tables over all variants
   DevGenome genome, scratch;
 
+  // An allocation has failed: screens take no more memory than they hold until
+  // a genome is loaded (a try for each search would free, fail and wait for the
+  // device each time, and change the captured passes).
+  bool memory_short = false;
   DevBuf screen_windows;  // windows of a queue's candidates (ScreenList), used on `stream`
   DevBuf screen_items, screen_counts;  // candidates that passed a screen (ScreenList), used on `stream`
   DevBuf queue[2], qcounts, hits, hits_sorted, summary_counts, hit_count, sort_tmp, row_bytes, row_offsets, row_count, text, small,
@@ -291,6 +295,12 @@ void launch_group_compare(const cof_handle* h, const PatternGroup& g, uint32_t* 
 // added to *qc.
 void launch_group_scan(const cof_handle* h, const PatternGroup& g, uint64_t w0, uint64_t w1, unsigned long long* qc,
                        const HitSink& sink);
+// b.ensure(bytes) for memory that a call cannot do without: where there is not
+// enough, once more after give_back.  On the thread that launches the screens.
+cudaError_t need(cof_handle* h, DevBuf& b, size_t bytes);
+// Frees the buffers of ensure_screen_list that only speed depends on (false:
+// there are none).  Launches queued so far are waited for.
+bool give_back(cof_handle* h);
 // The list buffers of the screens of launches over up to `positions` starts
 // (with `windows`, those of a queue's windows too).
 cof_status ensure_screen_list(cof_handle* h, uint64_t positions, bool windows);

@@ -132,6 +132,7 @@ struct cof_server {
   // finisher hand-off (under mu); the finisher drains until the worker is gone
   std::deque<ReqPtr> to_finish;
   bool worker_gone = false;
+  bool spare_wanted = false;  // the finisher is short of memory: the worker gives the screens' buffers back (give_back)
 
   // worker-only state
   std::unique_ptr<TableSet> tables;
@@ -243,19 +244,23 @@ cof_status run_step(cof_server* s, uint64_t k) {
   const GenomeView gv = h->genome.view();
   const uint64_t n = h->genome.n;
   uint64_t cap = std::max<uint64_t>(s->step_hits.cap / 8, 1u << 16);
-  COF_CUDA(h, s->step_hits.ensure(cap * 8));
-  COF_CUDA(h, s->step_count.ensure(8));
+  COF_CUDA(h, need(h, s->step_hits, cap * 8));
+  COF_CUDA(h, need(h, s->step_count, 8));
   const size_t nq = std::max<size_t>(T.groups.size(), 1) * (size_t)k;
-  COF_CUDA(h, h->qcounts.ensure(PassCounts::bytes(nq)));
+  COF_CUDA(h, need(h, h->qcounts, PassCounts::bytes(nq)));
   const PassCounts pc(h->qcounts, nq);
   // at most two oriented candidates per start position of a segment
-  COF_CUDA(h, h->queue[0].ensure(2 * s->seg_words * 32 * 4));
-  COF_CUDA(h, h->queue[1].ensure(2 * s->seg_words * 32 * 4));
-  const bool windows = std::any_of(T.groups.begin(), T.groups.end(), [](const PatternGroup& g) { return g.windows(); });
-  cof_status ls = ensure_screen_list(h, std::min<uint64_t>(n, s->seg_words * 32), windows);
-  if (ls) return ls;
+  COF_CUDA(h, need(h, h->queue[0], 2 * s->seg_words * 32 * 4));
+  COF_CUDA(h, need(h, h->queue[1], 2 * s->seg_words * 32 * 4));
+  bool screens = false, windows = false;
+  for (const PatternGroup& g : T.groups) {
+    screens |= g.screen_on;
+    windows |= g.windows();
+  }
   uint64_t count = 0;
   for (;;) {
+    cof_status ls = screens ? ensure_screen_list(h, std::min<uint64_t>(n, s->seg_words * 32), windows) : COF_OK;
+    if (ls) return ls;
     COF_CUDA(h, cudaMemsetAsync(h->qcounts.p, 0, PassCounts::bytes(nq), h->stream));
     COF_CUDA(h, cudaMemsetAsync(s->step_count.p, 0, 8, h->stream));
     COF_CUDA(h, cudaEventRecord(h->ev_start, h->stream));
@@ -295,19 +300,19 @@ cof_status run_step(cof_server* s, uint64_t k) {
       return fail(h, COF_ERR_NOMEM, "one ring step found " + std::to_string(count) +
                                         " hits, more than the hit buffer budget allows");
     cap = count + count / 8;
-    COF_CUDA(h, s->step_hits.ensure(cap * 8));
+    COF_CUDA(h, need(h, s->step_hits, cap * 8));
   }
   if (count) {
     // Sort the step's hits: each request's ids are one consecutive range, so
     // its hits become one run, appended to the request's own device buffer.
     const size_t A = T.reqs.size();
-    COF_CUDA(h, s->step_sorted.ensure(count * 8));
-    COF_CUDA(h, s->step_bounds.ensure((A + 1) * 8));
-    COF_CUDA(h, s->step_gid0.ensure((A + 1) * 4));
+    COF_CUDA(h, need(h, s->step_sorted, count * 8));
+    COF_CUDA(h, need(h, s->step_bounds, (A + 1) * 8));
+    COF_CUDA(h, need(h, s->step_gid0, (A + 1) * 4));
     size_t tmp = 0;
     COF_CUDA(h, cub::DeviceRadixSort::SortKeys(nullptr, tmp, s->step_hits.as<uint64_t>(),
                                                s->step_sorted.as<uint64_t>(), (int64_t)count, 0, 64, h->stream));
-    COF_CUDA(h, s->sort_tmp.ensure(tmp));
+    COF_CUDA(h, need(h, s->sort_tmp, tmp));
     tmp = s->sort_tmp.cap;
     COF_CUDA(h, cub::DeviceRadixSort::SortKeys(s->sort_tmp.p, tmp, s->step_hits.as<uint64_t>(),
                                                s->step_sorted.as<uint64_t>(), (int64_t)count, 0, 64, h->stream));
@@ -327,7 +332,7 @@ cof_status run_step(cof_server* s, uint64_t k) {
       if (!k || r.ran) continue;
       if ((r.n_hits + k) * 8 > r.hits.cap) {  // grow by doubling, keeping the hits so far
         DevBuf bigger(h->stream);
-        COF_CUDA(h, bigger.ensure(std::max<uint64_t>((r.n_hits + k) * 8, 2 * r.hits.cap)));
+        COF_CUDA(h, need(h, bigger, std::max<uint64_t>((r.n_hits + k) * 8, 2 * r.hits.cap)));
         if (r.n_hits)
           COF_CUDA(h, cudaMemcpyAsync(bigger.p, r.hits.p, r.n_hits * 8, cudaMemcpyDeviceToDevice, h->stream));
         r.hits = std::move(bigger);  // the old buffer is freed in stream order
@@ -335,7 +340,7 @@ cof_status run_step(cof_server* s, uint64_t k) {
       dst[a] = r.hits.as<uint64_t>() + r.n_hits;
       r.n_hits += k;
     }
-    COF_CUDA(h, s->step_dst.ensure(A * sizeof(uint64_t*)));
+    COF_CUDA(h, need(h, s->step_dst, A * sizeof(uint64_t*)));
     COF_CUDA(h, cudaMemcpyAsync(s->step_bounds.p, start.data(), (A + 1) * 8, cudaMemcpyHostToDevice, h->stream));
     COF_CUDA(h, cudaMemcpyAsync(s->step_dst.p, dst.data(), A * sizeof(uint64_t*), cudaMemcpyHostToDevice, h->stream));
     launch_scatter_runs(s->step_sorted.as<uint64_t>(), count, s->step_gid0.as<uint32_t>(),
@@ -344,6 +349,25 @@ cof_status run_step(cof_server* s, uint64_t k) {
   }
   s->steps += k;
   return COF_OK;
+}
+
+// need() on the finisher's thread: the worker, whose launches use the screens'
+// buffers, gives them back between two steps.
+cudaError_t finisher_need(cof_server* s, DevBuf& b, size_t bytes) {
+  const cudaError_t e = b.ensure(bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  {
+    std::unique_lock<std::mutex> lock(s->mu);
+    s->spare_wanted = true;
+    s->cv_work.notify_all();
+    s->cv_finish.wait(lock, [&] { return !s->spare_wanted || s->worker_gone; });
+    if (s->spare_wanted) give_back(s->h);
+    s->spare_wanted = false;
+  }
+  const cudaError_t again = b.ensure(bytes);
+  if (again != cudaSuccess) cudaGetLastError();
+  return again;
 }
 
 // CUDA check for the finisher: reports through `err`, not the handle.
@@ -386,16 +410,16 @@ cof_status format_batch(cof_server* s, const std::vector<ReqPtr>& rs, std::strin
   std::vector<ShapeFmt> sf;
   std::string pool;
   for (const ReqPtr& r : rs) append_format_tables(r->job, vf, sf, pool);
-  COF_FIN(s->fmt_vf.ensure(vf.size() * sizeof(VariantFmt)));
-  COF_FIN(s->fmt_sf.ensure(std::max<size_t>(sf.size(), 1) * sizeof(ShapeFmt)));
-  COF_FIN(s->fmt_pool.ensure(std::max<size_t>(pool.size(), 1)));
-  COF_FIN(s->fmt_in.ensure(nh * 8));
-  COF_FIN(s->fmt_hits.ensure(nh * 8));
-  COF_FIN(s->fmt_bytes.ensure(nh * 8));
-  COF_FIN(s->fmt_off.ensure(nh * 8));
-  COF_FIN(s->fmt_cnt.ensure(nh * 4));
-  COF_FIN(s->fmt_gid0.ensure(k * 4));
-  COF_FIN(s->fmt_bounds.ensure((k + 1) * 8));
+  COF_FIN(finisher_need(s, s->fmt_vf, vf.size() * sizeof(VariantFmt)));
+  COF_FIN(finisher_need(s, s->fmt_sf, std::max<size_t>(sf.size(), 1) * sizeof(ShapeFmt)));
+  COF_FIN(finisher_need(s, s->fmt_pool, std::max<size_t>(pool.size(), 1)));
+  COF_FIN(finisher_need(s, s->fmt_in, nh * 8));
+  COF_FIN(finisher_need(s, s->fmt_hits, nh * 8));
+  COF_FIN(finisher_need(s, s->fmt_bytes, nh * 8));
+  COF_FIN(finisher_need(s, s->fmt_off, nh * 8));
+  COF_FIN(finisher_need(s, s->fmt_cnt, nh * 4));
+  COF_FIN(finisher_need(s, s->fmt_gid0, k * 4));
+  COF_FIN(finisher_need(s, s->fmt_bounds, (k + 1) * 8));
   COF_FIN(cudaMemcpyAsync(s->fmt_vf.p, vf.data(), vf.size() * sizeof(VariantFmt), cudaMemcpyHostToDevice, st));
   if (!sf.empty())
     COF_FIN(cudaMemcpyAsync(s->fmt_sf.p, sf.data(), sf.size() * sizeof(ShapeFmt), cudaMemcpyHostToDevice, st));
@@ -418,7 +442,7 @@ cof_status format_batch(cof_server* s, const std::vector<ReqPtr>& rs, std::strin
                                          (int64_t)nh, 7, end_bit, st));
   COF_FIN(cub::DeviceScan::ExclusiveSum(nullptr, t1, s->fmt_bytes.as<uint64_t>(), s->fmt_off.as<uint64_t>(),
                                         (int64_t)nh, st));
-  COF_FIN(s->fmt_tmp.ensure(std::max(t0, t1)));
+  COF_FIN(finisher_need(s, s->fmt_tmp, std::max(t0, t1)));
   t0 = s->fmt_tmp.cap;
   COF_FIN(cub::DeviceRadixSort::SortKeys(s->fmt_tmp.p, t0, s->fmt_in.as<uint64_t>(), s->fmt_hits.as<uint64_t>(),
                                          (int64_t)nh, 7, end_bit, st));
@@ -435,7 +459,7 @@ cof_status format_batch(cof_server* s, const std::vector<ReqPtr>& rs, std::strin
   COF_FIN(cudaMemcpyAsync(bounds.data(), s->fmt_bounds.p, (k + 1) * 8, cudaMemcpyDeviceToHost, st));
   COF_FIN(cudaStreamSynchronize(st));
   const uint64_t bytes = bounds[k];
-  COF_FIN(s->fmt_text.ensure(bytes + 1));
+  COF_FIN(finisher_need(s, s->fmt_text, bytes + 1));
   launch_write_rows(gv, ft, s->fmt_hits.as<uint64_t>(), nh, s->fmt_off.as<uint64_t>(), 0, bytes,
                     s->fmt_text.as<char>(), st);
   COF_FIN(cudaGetLastError());
@@ -548,7 +572,12 @@ void worker_main(cof_server* s) {
     std::unique_ptr<TableSet> fresh;
     {
       std::unique_lock<std::mutex> lock(s->mu);
-      s->cv_work.wait(lock, [&] { return s->stop || admissible(s) || s->built || tables_live(s); });
+      s->cv_work.wait(lock, [&] { return s->stop || s->spare_wanted || admissible(s) || s->built || tables_live(s); });
+      if (s->spare_wanted) {
+        give_back(h);
+        s->spare_wanted = false;
+        s->cv_finish.notify_all();
+      }
       if (s->stop) break;
       // Admit waiting requests while the variant budget allows (always at
       // least one, so a request larger than the budget still runs alone).

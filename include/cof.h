@@ -205,7 +205,10 @@ cof_status cof_server_set_step_segments(cof_server* s, uint32_t segments);
  * 32 KiB per compare variant, at least 1 MiB and at most 64 MiB. */
 cof_status cof_server_set_hit_reserve(cof_server* s, uint64_t bytes);
 /* Device bytes of request hit buffers after the latest ring step, their
- * maximum so far, and the bytes of the two shared candidate queues. */
+ * maximum so far, and the bytes of the two shared candidate queues.  Requests
+ * that a table screen searches share its list and windows too (up to 1.5 GiB,
+ * less where memory is short, freed when other allocations need the memory):
+ * these are not counted. */
 cof_status cof_server_memory(cof_server* s, uint64_t* held_hit_bytes, uint64_t* max_held_hit_bytes,
                              uint64_t* queue_bytes);
 const char* cof_server_last_error(cof_server* s);

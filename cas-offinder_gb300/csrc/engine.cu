@@ -41,7 +41,6 @@ using namespace cof::eng;
 std::mutex g_open_mu;
 std::string g_open_err;
 
-// Uploads a packed genome into `dg` (copies are stream-ordered on h->stream).
 // Queues the copies of streamed-upload chunks [issued, upto) on h->stream2,
 // the finders' stream: each finder follows the copies queued before it.
 cof_status issue_upload(cof_handle* h, size_t upto) {
@@ -113,6 +112,7 @@ size_t upload_chunk_of(const cof_handle* h, uint64_t w1) {
   return std::lower_bound(h->upload_ends.begin(), h->upload_ends.end(), need) - h->upload_ends.begin();
 }
 
+// Uploads a packed genome into `dg` (copies are stream-ordered on h->stream).
 // With `streamed` the planes are copied under the search: page-locked ones
 // (h->upload_pinned) are queued here (queue_upload_ahead), others by
 // run_passes (issue_upload).  The host planes must stay valid until both that

@@ -73,7 +73,7 @@ struct ScreenPlan {
   ScreenGeom geom;
   std::vector<uint32_t> records;  // screen_record_words(nw) per variant
   std::vector<uint32_t> first;    // words * (fields + 1): first record of each class of a word, then the word's end
-  uint32_t level = 0;             // the partition taken (index of screen_levels)
+  uint32_t level = 0;             // the partition taken (screen_level_name)
   std::vector<uint32_t> candidates;  // levels worth timing, the model's best first
   bool windows() const;  // it extracts the queue's windows first
 };
@@ -92,7 +92,7 @@ struct HitCosts {
   double direct, counted;
 };
 HitCosts hit_costs(const std::vector<const Variant*>& vars, const ScreenPlan& plan);
-// Text of a partition ("2/guide", "4 guides", ...).
+// Text of a partition ("2 classes/guide", "4 guides/class", ...).
 const char* screen_level_name(uint32_t level);
 
 // Candidates that passed a class, listed per warp of the screening launch: an
